@@ -30,9 +30,10 @@ EMPTY, ELECTRON, HOLE, DEFECT, SOURCE, DRAIN = range(6)
 def reference_tree():
     """The reference source tree the compiled-reference recipes read: the
     REFERENCE environment variable, else the tree's usual mount point; None
-    where neither holds it (a GPU box has no copy)."""
+    where neither holds its sources (a GPU box has no copy, and a mount point
+    may be empty)."""
     path = os.environ.get("REFERENCE", "/root/reference")
-    return path if os.path.isdir(path) else None
+    return path if os.path.isfile(os.path.join(path, "src", "langmuirCore", "kernel.cl")) else None
 
 
 def build(ref: bool = False) -> None:
