@@ -16,6 +16,7 @@
 #include "langmuir_b200.h"
 #include "lgm_context.hpp"
 #include "lgm_cull.cuh"
+#include "lgm_mma.cuh"
 
 using namespace lgm;
 
@@ -78,22 +79,31 @@ lgm_status grow_host(lgm_ctx* c, T** p, size_t* cap, size_t need) {
 // deterministic.  bins_end[b] is the end of bin b after the scatter.  Entries
 // n .. n_pad-1 are zero-charge padding at the origin; their weight is
 // (q*m) * y = 0 * finite = 0.
-__device__ __forceinline__ void source_record(int sj, int qj, int X, int XY, int Y, int volume,
-                                              float4* __restrict__ geo, float2* __restrict__ qq,
-                                              int dst, unsigned* err) {
-    float a = 0.f, b = 0.f, cc = 0.f, d = -0.5f, qf = 0.f;
-    if (sj < 0 || sj >= volume) {
-        atomicOr(err, DEVERR_SOURCE_RANGE);
-    } else {
-        // Grid::getIndexX/Y/Z (cubicgrid.cpp:132-145), as kernel.cl:266-268.
-        const int z = sj / XY, y = sj / X - z * Y, x = sj % X;
-        a = -2.f * x; b = -2.f * y; cc = -2.f * z;
-        d = (float)(x * x + y * y + z * z) - 0.5f;
-        qf = (float)qj;
+//
+// fmt selects the records a call's pair kernel reads: kFmtFloat (the FP32 and
+// FP64 tiles), kFmtHalf (the tensor-core sums), or both (the autotuner).
+constexpr int kFmtFloat = 1, kFmtHalf = 2;
+struct Records {
+    int fmt;
+    float4* geo;
+    float2* qq;
+    float4* tgt;
+    uint32_t* frag;
+    float* q1;
+    uint4* tgt16;
+};
+
+// The record of one source at slot dst; empty: a zero-charge record at the origin.
+__device__ __forceinline__ void write_source(const Records& R, int dst, int x, int y, int z,
+                                             float q) {
+    if (R.fmt & kFmtFloat) {
+        const float a = -2.f * x, b = -2.f * y, c = -2.f * z;
+        const float d = (float)(x * x + y * y + z * z) - 0.5f;
+        R.geo[2 * dst] = make_float4(a, a, b, b);
+        R.geo[2 * dst + 1] = make_float4(c, c, d, d);
+        R.qq[dst] = make_float2(q, q);
     }
-    geo[2 * dst] = make_float4(a, a, b, b);
-    geo[2 * dst + 1] = make_float4(cc, cc, d, d);
-    qq[dst] = make_float2(qf, qf);
+    if (R.fmt & kFmtHalf) store_source(R.frag, R.q1, dst, x, y, z, q);
 }
 
 __device__ __forceinline__ void prep_source(const int j, const int32_t* __restrict__ s,
@@ -101,13 +111,12 @@ __device__ __forceinline__ void prep_source(const int j, const int32_t* __restri
                                             const int32_t* __restrict__ key,
                                             const int32_t* __restrict__ tmp,
                                             const int32_t* __restrict__ bins_end, int X, int Y,
-                                            int XY, int volume, float4* __restrict__ geo,
-                                            float2* __restrict__ qq, unsigned* err) {
-    if (j >= n_pad) return;
+                                            int XY, int volume, const Records& R, unsigned* err) {
+    // (one more group of padding, behind the last chunk: lgm_mma.cuh's pad_group)
+    if (j >= n_pad + kGroup || (j >= n_pad && !(R.fmt & kFmtHalf))) return;
     if (j >= n) {
-        geo[2 * j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        geo[2 * j + 1] = make_float4(0.f, 0.f, -0.5f, -0.5f);
-        qq[j] = make_float2(0.f, 0.f);
+        if (j < n_pad) write_source(R, j, 0, 0, 0, 0.f);
+        else store_source(R.frag, R.q1, j, 0, 0, 0, 0.f);
         return;
     }
     const int i = tmp[j];
@@ -120,7 +129,14 @@ __device__ __forceinline__ void prep_source(const int j, const int32_t* __restri
         const int so = s[o];
         rank += (so < si) | ((so == si) & (o < i));
     }
-    source_record(si, q[i], X, XY, Y, volume, geo, qq, lo + rank, err);
+    if (si < 0 || si >= volume) {
+        atomicOr(err, DEVERR_SOURCE_RANGE);
+        write_source(R, lo + rank, 0, 0, 0, 0.f);
+    } else {
+        // Grid::getIndexX/Y/Z (cubicgrid.cpp:132-145), as kernel.cl:266-268.
+        const int z = si / XY, y = si / X - z * Y, x = si % X;
+        write_source(R, lo + rank, x, y, z, (float)q[i]);
+    }
 }
 
 // Physical targets: for each requested term the (possibly mirrored) target
@@ -134,7 +150,7 @@ __device__ __forceinline__ void prep_target(const int j, const int32_t* __restri
                                             const int32_t* __restrict__ tkey,
                                             const int32_t* __restrict__ ttmp,
                                             const int32_t* __restrict__ bins_end,
-                                            int32_t* __restrict__ perm, float4* __restrict__ tgt,
+                                            int32_t* __restrict__ perm, const Records& R,
                                             unsigned* err) {
     if (j >= t_pad) return;  // j: the scatter slot
     // The target scattered to slot j goes to physical slot g: its bin's start
@@ -177,11 +193,13 @@ __device__ __forceinline__ void prep_target(const int j, const int32_t* __restri
         int xp = x;
         if (term == 1) xp = -1 - x;
         if (term == 2) xp = 2 * X - 1 - x;
-        const float fx = (float)xp, fy = (float)y, fz = (float)z;
-        // padding slots (g >= t) carry w = -1: the cull leaves them out of the
-        // tiles' boxes, and their sums are never read
-        tgt[(size_t)slot * t_pad + g] =
-            make_float4(fx, fy, fz, g < t ? (float)(xp * xp + y * y + z * z) : -1.f);
+        // padding slots (g >= t) carry a mark (w = -1): the cull leaves them
+        // out of the tiles' boxes, and their sums are never read
+        if (R.fmt & kFmtFloat)
+            R.tgt[(size_t)slot * t_pad + g] =
+                make_float4((float)xp, (float)y, (float)z,
+                            g < t ? (float)(xp * xp + y * y + z * z) : -1.f);
+        if (R.fmt & kFmtHalf) R.tgt16[(size_t)slot * t_pad + g] = target_row(xp, y, z, g >= t);
         ++slot;
     }
 }
@@ -193,20 +211,19 @@ __global__ void prep_records(int tb, const int32_t* __restrict__ ts, int t, int 
                              int shift, const int32_t* __restrict__ tkey,
                              const int32_t* __restrict__ ttmp,
                              const int32_t* __restrict__ tbins_end, int32_t* __restrict__ perm,
-                             float4* __restrict__ tgt, const int32_t* __restrict__ s,
+                             const Records R, const int32_t* __restrict__ s,
                              const int32_t* __restrict__ q, int n, int n_pad,
                              const int32_t* __restrict__ skey, const int32_t* __restrict__ stmp,
-                             const int32_t* __restrict__ sbins_end, float4* __restrict__ geo,
-                             float2* __restrict__ qq, unsigned* err) {
+                             const int32_t* __restrict__ sbins_end, unsigned* err) {
     pdl_wait();
     pdl_trigger();
     const int b = (int)blockIdx.x;
     if (b < tb)
         prep_target(b * (int)blockDim.x + (int)threadIdx.x, ts, t, t_pad, all_sites, terms, X, Y,
-                    XY, volume, shift, tkey, ttmp, tbins_end, perm, tgt, err);
+                    XY, volume, shift, tkey, ttmp, tbins_end, perm, R, err);
     else
         prep_source((b - tb) * (int)blockDim.x + (int)threadIdx.x, s, q, n, n_pad, skey, stmp,
-                    sbins_end, X, Y, XY, volume, geo, qq, err);
+                    sbins_end, X, Y, XY, volume, R, err);
 }
 
 // The last kernel of a call clears both bin arrays (their last reader,
@@ -455,6 +472,7 @@ struct Variant {
     PairFn fn[4];
     CulledFn cfn[4];  // [3]: the FP64-table path (culled variants only)
     int ws = 0;       // warp-specialised culled kernel: its stages (0: not)
+    int tc = 0;       // r^2 on the tensor cores (lgm_mma.cuh): FP16 records
 };
 #define LGM_VARIANT_S(NT, RP, SUB, SK)                                                    \
     Variant {                                                                             \
@@ -494,6 +512,15 @@ struct Variant {
              &pair_kernel_culled_ws<0, 2, NW, RP, SUB, S, MINB>},                             \
             S                                                                                 \
     }
+// r^2 on the tensor cores: warps of 32 targets, items of about three chunks
+#define LGM_VARIANT_MMA                                                                      \
+    Variant {                                                                                 \
+        kMmaThreads, 1, kGroup, 1, 1, kItemGroups / kGroupsPerChunk,                          \
+            {nullptr, nullptr, nullptr, nullptr},                                             \
+            {&pair_kernel_mma<0, 0, kMmaTabPoint>, &pair_kernel_mma<1, 0, kMmaTabGauss>,      \
+             &pair_kernel_mma<0, 1, 8>, &pair_kernel_mma<0, 2, 8>},                           \
+            0, 1                                                                              \
+    }
 const Variant kVariants[] = {
     LGM_VARIANT(128, 4, 16),       LGM_VARIANT(128, 4, 8),        LGM_VARIANT(128, 2, 16),
     LGM_VARIANT(128, 8, 16),       LGM_VARIANT(256, 4, 16),       LGM_VARIANT(64, 4, 16),
@@ -519,6 +546,7 @@ const Variant kVariants[] = {
     // one vote per 2 or 4 sources, or none
     LGM_VARIANT_CULL_WSV(4, 2, 16, 2, 4, 4, 2), LGM_VARIANT_CULL_WSV(4, 2, 16, 2, 4, 4, 0),
     LGM_VARIANT_CULL_WSV(4, 2, 16, 2, 4, 4, 4),
+    LGM_VARIANT_MMA,
 };
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 static_assert(kNumVariants <= (int)(sizeof(lgm_ctx::bps) / sizeof(lgm_ctx::bps[0])),
@@ -526,20 +554,33 @@ static_assert(kNumVariants <= (int)(sizeof(lgm_ctx::bps) / sizeof(lgm_ctx::bps[0
 // warp-specialised culled, 4 target warps, 2 target pairs, runs of 16, 2
 // chunks per item, one vote per 2 sources (2% faster than a vote per source
 // on the 256x256x16 and 128x128x64 workloads, the same bits)
-constexpr int kDefaultVariant = 32;
+// r^2 on the tensor cores
+constexpr int kDefaultVariant = kNumVariants - 1;
 
-const void* kernel_of(const Variant& V, int fi) {
-    return V.cull ? reinterpret_cast<const void*>(V.cfn[fi])
+// The culled kernel of variant V for path index fi and cutoff^2 c2.
+CulledFn culled_fn(const Variant& V, int fi, int c2) {
+    if (V.tc && fi < 2 && c2 > kMmaTabEntries)
+        return fi == 0 ? &pair_kernel_mma<0, 0, 0> : &pair_kernel_mma<1, 0, 0>;
+    return V.cfn[fi];
+}
+const void* kernel_of(const Variant& V, int fi, int c2) {
+    return V.cull ? reinterpret_cast<const void*>(culled_fn(V, fi, c2))
                   : reinterpret_cast<const void*>(V.fn[fi]);
 }
 
 // Threads of a CTA (a warp-specialised variant adds its producer warp) and
 // dynamic shared memory for path index fi with table entries 0 .. tab_k.
 int variant_threads(const Variant& V) { return V.nt + (V.ws ? 32 : 0); }
-size_t variant_smem(const Variant& V, int fi, int tab_k) {
+size_t variant_smem(const Variant& V, int fi, int tab_k, int c2) {
+    if (V.tc) return mma_smem_bytes(fi < 2 && c2 <= kMmaTabEntries ? c2 : tab_k + 1, fi == 3 ? 8 : 4);
     if (V.ws) return ws_smem_bytes(V.ws, tab_k, fi == 3 ? 8 : 4);
     return fi == 3 ? pair_smem_bytes64(tab_k) : pair_smem_bytes(tab_k);
 }
+
+// Targets of a tile.  (The tensor-core variant's is a warp's 32 targets; its
+// target_pairs reads 1.)
+int variant_tile(const Variant& V) { return V.tc ? kSeg : V.nt * 2 * V.rp; }
+int variant_targets_per_thread(const Variant& V) { return V.tc ? 1 : 2 * V.rp; }
 
 int fn_index(int kind, int path) {
     if (path == LGM_PATH_TABLE64) return 3;  // one kernel: the table holds w for the kind
@@ -573,14 +614,24 @@ Shape shape_of(int n, int t, unsigned terms) {
 }
 
 lgm_status prep(lgm_ctx* c, unsigned terms, const int32_t* d_src, const int32_t* d_q, int n,
-                const int32_t* d_tgt_site, int t, int all_sites, const Shape& sh,
+                const int32_t* d_tgt_site, int t, int all_sites, const Shape& sh, int fmt,
                 cudaStream_t st) {
     const lgm_config& cf = c->cfg;
     lgm_status s;
-    if ((s = grow_device(c, &c->d_geo, &c->geo_cap, (size_t)sh.n_pad * 2)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_qq, &c->qq_cap, (size_t)sh.n_pad)) != LGM_OK) return s;
-    // room for the widest target tile of any variant
-    if ((s = grow_device(c, &c->d_tgt, &c->tgt_cap, (size_t)sh.t_phys + 4096)) != LGM_OK) return s;
+    // target records: room for the widest target tile of any variant
+    const size_t tgt_n = (size_t)sh.t_phys + 4096;
+    if (fmt & kFmtFloat) {
+        if ((s = grow_device(c, &c->d_geo, &c->geo_cap, (size_t)sh.n_pad * 2)) != LGM_OK) return s;
+        if ((s = grow_device(c, &c->d_qq, &c->qq_cap, (size_t)sh.n_pad)) != LGM_OK) return s;
+        if ((s = grow_device(c, &c->d_tgt, &c->tgt_cap, tgt_n)) != LGM_OK) return s;
+    }
+    if (fmt & kFmtHalf) {
+        const size_t ns = (size_t)sh.n_pad + kGroup;
+        if ((s = grow_device(c, &c->d_frag, &c->frag_cap, ns * 4)) != LGM_OK) return s;
+        if ((s = grow_device(c, &c->d_q1, &c->q1_cap, ns)) != LGM_OK) return s;
+        if ((s = grow_device(c, &c->d_tgt16, &c->tgt16_cap, tgt_n)) != LGM_OK) return s;
+    }
+    const Records R{fmt, c->d_geo, c->d_qq, c->d_tgt, c->d_frag, c->d_q1, c->d_tgt16};
     if ((s = grow_device(c, &c->d_key, &c->key_cap, (size_t)t)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_perm, &c->perm_cap, (size_t)t)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_ttmp, &c->ttmp_cap, (size_t)t)) != LGM_OK) return s;
@@ -601,12 +652,11 @@ lgm_status prep(lgm_ctx* c, unsigned terms, const int32_t* d_src, const int32_t*
                              c->d_skey, c->d_sbins, c->d_bins + 2 * c->bins_stride));
     LGM_CUDA(c, launch_chain(ov, scatter_both, tb, 256, 0, st, c->d_key, t, c->d_bins, c->d_ttmp,
                              c->d_skey, n, c->d_sbins, c->d_stmp));
-    const int ptb = (sh.t_pad + 255) / 256, psb = (sh.n_pad + 255) / 256;
+    const int ptb = (sh.t_pad + 255) / 256, psb = (sh.n_pad + kGroup + 255) / 256;
     LGM_CUDA(c, launch_chain(ov, prep_records, ptb + psb, 256, 0, st, ptb, d_tgt_site, t, sh.t_pad,
                              all_sites, terms, cf.grid_x, cf.grid_y, c->xy, c->volume,
-                             c->cell_shift, c->d_key, c->d_ttmp, c->d_bins, c->d_perm, c->d_tgt,
-                             d_src, d_q, n, sh.n_pad, c->d_skey, c->d_stmp, c->d_sbins, c->d_geo,
-                             c->d_qq, c->d_err));
+                             c->cell_shift, c->d_key, c->d_ttmp, c->d_bins, c->d_perm, R, d_src,
+                             d_q, n, sh.n_pad, c->d_skey, c->d_stmp, c->d_sbins, c->d_err));
     return LGM_OK;
 }
 
@@ -634,24 +684,31 @@ lgm_status launch_culled(lgm_ctx* c, int kind, int v, const Shape& sh, const Pai
                          cudaStream_t st, int* splits_out) {
     const Variant& V = kVariants[v];
     const int fi = fn_index(kind, c->cfg.path);
-    const int TS = V.nt * 2 * V.rp;
+    const int TS = variant_tile(V);
     const int tiles = (sh.t_phys + TS - 1) / TS;
-    const int max_items = std::min(kMaxItemsPerTile, (sh.n_chunks + V.per_item - 1) / V.per_item);
+    const int grid = c->sm_count * std::max(1, c->bps[v][fi]);
+    int per_item = V.per_item, max_items = kMaxItemsPerTile;
+    if (V.tc) mma_items(tiles, sh.n_chunks * kGroupsPerChunk, false, &per_item, &max_items);
+    else max_items = std::max(1, std::min(max_items, (sh.n_chunks + per_item - 1) / per_item));
+    const int mask_stride = (sh.n_chunks + 31) / 32 * 32;
     if (V.nt / 32 > kMaxSegments) return fail(c, LGM_ERR_STATE, "culled variant wider than the cull");
-    const size_t item_cap = (size_t)tiles * std::max(1, max_items);
+    const size_t item_cap = (size_t)tiles * max_items;
     lgm_status s;
     if ((s = grow_device(c, &c->d_cbox, &c->cbox_cap, (size_t)sh.n_chunks)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_gbox, &c->gbox_cap, (size_t)sh.n_chunks * kGroupsPerChunk)) !=
         LGM_OK)
         return s;
-    if ((s = grow_device(c, &c->d_live, &c->live_cap, (size_t)tiles * sh.n_chunks)) != LGM_OK)
-        return s;
+    if (V.tc) s = grow_device(c, &c->d_gmask, &c->gmask_cap, (size_t)tiles * mask_stride);
+    else s = grow_device(c, &c->d_live, &c->live_cap, (size_t)tiles * sh.n_chunks);
+    if (s != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_items, &c->items_cap, item_cap)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_tile_first, &c->tfirst_cap, (size_t)tiles)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_tile_items, &c->titems_cap, (size_t)tiles)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_part, &c->part_cap, item_cap * TS)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_order, &c->order_cap, item_cap)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_oitems, &c->oitems_cap, item_cap)) != LGM_OK) return s;
+    if (!V.tc) {
+        if ((s = grow_device(c, &c->d_order, &c->order_cap, item_cap)) != LGM_OK) return s;
+        if ((s = grow_device(c, &c->d_oitems, &c->oitems_cap, item_cap)) != LGM_OK) return s;
+    }
     PairArgs P = A;
     P.part = c->d_part;
     CullArgs C;
@@ -662,9 +719,13 @@ lgm_status launch_culled(lgm_ctx* c, int kind, int v, const Shape& sh, const Pai
     C.t_phys = sh.t_phys;
     C.c2 = c->cfg.electrostatic_cutoff * c->cfg.electrostatic_cutoff;
     C.tile_size = TS;
-    C.per_item = V.per_item;
-    C.max_items = std::max(1, max_items);
+    C.per_item = per_item;
+    C.max_items = max_items;
     C.live = c->d_live;
+    C.tgt16 = c->d_tgt16;
+    C.gmask = c->d_gmask;
+    C.mask_stride = mask_stride;
+    C.max_tiles = tiles;
     C.live_stride = sh.n_chunks;
     C.items = c->d_items;
     C.item_count = c->d_item_count;
@@ -683,17 +744,22 @@ lgm_status launch_culled(lgm_ctx* c, int kind, int v, const Shape& sh, const Pai
         c->count_pending = true;
     }
     const bool ov = c->overlap;
-    LGM_CUDA(c, launch_chain(ov, chunk_boxes_kernel, sh.n_chunks, CH, 0, st, P, C));
-    // its last block orders the items
-    LGM_CUDA(c, launch_chain(ov, cull_kernel, tiles, kCullThreads, 0, st, C));
+    if (V.tc) {
+        LGM_CUDA(c, launch_chain(ov, chunk_boxes_mma_kernel, sh.n_chunks, CH, 0, st, P, C));
+        LGM_CUDA(c, launch_chain(ov, cull_mma_kernel, (tiles + kCullSegs - 1) / kCullSegs,
+                                 kCullThreads, 0, st, C));
+    } else {
+        LGM_CUDA(c, launch_chain(ov, chunk_boxes_kernel, sh.n_chunks, CH, 0, st, P, C));
+        // its last block orders the items
+        LGM_CUDA(c, launch_chain(ov, cull_kernel, tiles, kCullThreads, 0, st, C));
+    }
     // timing on: the events bracket the pair kernel alone (recorded again here)
     if (c->timing) LGM_CUDA(c, cudaEventRecord(c->ev_pair0, st));
-    const int grid = c->sm_count * std::max(1, c->bps[v][fi]);
-    LGM_CUDA(c, launch_chain(ov, V.cfn[fi], grid, variant_threads(V),
-                             variant_smem(V, fi, P.tab_k), st, P, C));
+    LGM_CUDA(c, launch_chain(ov, culled_fn(V, fi, C.c2), grid, variant_threads(V),
+                             variant_smem(V, fi, P.tab_k, C.c2), st, P, C));
     c->last.ctas = grid;
     c->last.threads = variant_threads(V);
-    c->last.targets_per_thread = 2 * V.rp;
+    c->last.targets_per_thread = variant_targets_per_thread(V);
     c->last.variant = v;
     c->last.splits = 0;
     *splits_out = 0;
@@ -708,6 +774,8 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int v, const Shape& sh, cudaStream_
         PairArgs A;
         A.geo = c->d_geo; A.qq = c->d_qq; A.n_chunks = sh.n_chunks; A.splits = 1;
         A.tgt = c->d_tgt; A.t_phys = sh.t_phys;
+        A.frag = c->d_frag; A.q1 = c->d_q1; A.tgt16 = c->d_tgt16;
+        A.pad_group = sh.n_chunks * kGroupsPerChunk;
         A.c2 = (float)(cf.electrostatic_cutoff * cf.electrostatic_cutoff);
         A.err = c->d_err;
         if (cf.path == LGM_PATH_TABLE64) {
@@ -784,8 +852,12 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         return LGM_OK;
     }
     const Shape sh = shape_of(n, t, terms);
+    const int v = choose_variant(c, kind, sh);
+    const int fmt =
+        cf.precision == LGM_PREC_FP64 || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
     lgm_status s;
-    if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, st)) != LGM_OK) return s;
+    if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, fmt, st)) != LGM_OK)
+        return s;
     int splits = 1;
     if (c->timing) LGM_CUDA(c, cudaEventRecord(c->ev_pair0, st));
     if (cf.precision == LGM_PREC_FP64) {
@@ -805,8 +877,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         c->last.threads = kF64Threads;
         c->last.targets_per_thread = 1;
     } else {
-        if ((s = launch_pair(c, kind, choose_variant(c, kind, sh), sh, st, &splits)) != LGM_OK)
-            return s;
+        if ((s = launch_pair(c, kind, v, sh, st, &splits)) != LGM_OK) return s;
     }
     if (c->timing) {
         LGM_CUDA(c, cudaEventRecord(c->ev_pair1, st));
@@ -823,7 +894,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     } else {
         const Variant& V = kVariants[c->last.variant];
         LGM_CUDA(c, launch_chain(c->overlap, finalize_items, (t + 31) / 32, dim3(32, 3), 0, st,
-                                 c->d_part, c->d_tile_first, c->d_tile_items, V.nt * 2 * V.rp, t,
+                                 c->d_part, c->d_tile_first, c->d_tile_items, variant_tile(V), t,
                                  sh.t_pad, sh.nterms, cf.electrostatic_prefactor, c->d_perm, d_out,
                                  c->d_bins, nbins, c->d_err, err_out));
         c->last.kernel_launches = 7;  // bins (+ scan), scatter, records, boxes, cull, pair, finalize
@@ -1103,25 +1174,25 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
         const int tab_of[4] = {0, c->gtab_k, std::max(c->rtab_k, c->gtab_k), c->rtab_k};
         for (int v = 0; v < kNumVariants; ++v)
             for (int fi = 0; fi < 4; ++fi) {
-                if (!kernel_of(kVariants[v], fi)) continue;
+                if (!kernel_of(kVariants[v], fi, c2)) continue;
                 // the table kernels serve only their own path
                 if (fi == 2 && cf.path != LGM_PATH_TABLE) continue;
                 if (fi == 3 && cf.path != LGM_PATH_TABLE64) continue;
-                const size_t smem = variant_smem(kVariants[v], fi, tab_of[fi]);
+                const size_t smem = variant_smem(kVariants[v], fi, tab_of[fi], c2);
                 if (smem > 48 * 1024) {
                     if (smem > (size_t)prop.sharedMemPerBlockOptin) {
                         g_create_error = "cutoff too large for the shared-memory tables";
                         lgm_destroy(c);
                         return LGM_ERR_UNSUPPORTED;
                     }
-                    if ((e = cudaFuncSetAttribute(kernel_of(kVariants[v], fi),
+                    if ((e = cudaFuncSetAttribute(kernel_of(kVariants[v], fi, c2),
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)smem)) != cudaSuccess)
                         return bail("cudaFuncSetAttribute", e);
                 }
                 int bps = 0;
                 if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                         &bps, kernel_of(kVariants[v], fi), variant_threads(kVariants[v]),
+                         &bps, kernel_of(kVariants[v], fi, c2), variant_threads(kVariants[v]),
                          smem)) != cudaSuccess)
                     return bail("cudaOccupancyMaxActiveBlocksPerMultiprocessor", e);
                 c->bps[v][fi] = bps;
@@ -1142,7 +1213,8 @@ lgm_status lgm_destroy(lgm_ctx* c) {
                         c->d_skey,  c->d_stmp,       c->d_cbox,       c->d_gbox,
                         c->d_live,  c->d_items,      c->d_tile_first, c->d_tile_items,
                         c->d_item_count, c->d_examined, c->d_rtab64,  c->d_gtab64,
-                        c->d_cost_hist,  c->d_order,     c->d_oitems};
+                        c->d_cost_hist,  c->d_order,     c->d_oitems,     c->d_frag,
+                        c->d_q1,         c->d_tgt16,     c->d_gmask};
     for (void* p : dev_ptrs)
         if (p) cudaFree(p);
     void* host_ptrs[] = {c->h_s, c->h_q, c->h_t, c->h_o, c->h_err};
@@ -1259,7 +1331,9 @@ lgm_status lgm_autotune(lgm_ctx* c, lgm_kind kind, uint32_t terms, int32_t n, in
     LGM_CUDA(c, cudaMemcpyAsync(c->d_q, hq.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
     LGM_CUDA(c, cudaMemcpyAsync(c->d_t, ht.data(), sizeof(int32_t) * t, cudaMemcpyHostToDevice, st));
     const Shape sh = shape_of(n, t, terms);
-    if ((s = prep(c, terms, c->d_s, c->d_q, n, c->d_t, t, 0, sh, st)) != LGM_OK) return s;
+    if ((s = prep(c, terms, c->d_s, c->d_q, n, c->d_t, t, 0, sh, kFmtFloat | kFmtHalf, st)) !=
+        LGM_OK)
+        return s;
     cudaEvent_t e0, e1;
     LGM_CUDA(c, cudaEventCreate(&e0));
     LGM_CUDA(c, cudaEventCreate(&e1));

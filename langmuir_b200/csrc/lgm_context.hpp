@@ -21,6 +21,11 @@ struct lgm_ctx {
     float4* d_geo = nullptr;  size_t geo_cap = 0;   // 2 float4 per source
     float2* d_qq = nullptr;   size_t qq_cap = 0;    // 1 float2 per source
     float4* d_tgt = nullptr;  size_t tgt_cap = 0;   // per physical target
+    // tensor-core sums (lgm_mma.cuh): source fragments, charges, target rows, live groups
+    uint32_t* d_frag = nullptr; size_t frag_cap = 0;
+    float* d_q1 = nullptr;    size_t q1_cap = 0;
+    uint4* d_tgt16 = nullptr; size_t tgt16_cap = 0;
+    uint8_t* d_gmask = nullptr; size_t gmask_cap = 0;
     double* d_part = nullptr; size_t part_cap = 0;  // split partial sums
     int32_t* d_s = nullptr;   size_t s_cap = 0;     // staging for host-buffer calls
     int32_t* d_q = nullptr;   size_t q_cap = 0;

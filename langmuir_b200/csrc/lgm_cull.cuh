@@ -125,29 +125,35 @@ struct CullArgs {
     // with order: culled tiles so far (zeroed by chunk_boxes block 0); the
     // cull's last block to finish writes order[]
     int* done = nullptr;
+    // Tensor-core sums (lgm_mma.cuh; a tile is a segment of 32 targets): FP16
+    // target rows, a byte of live groups per (segment, chunk), and for a batch
+    // the counter of the common item list and the problem of each of its items
+    const uint4* tgt16 = nullptr;
+    uint8_t* gmask = nullptr;         // [tiles][mask_stride]
+    int mask_stride = 0;
+    int max_tiles = 0;                // segments tile_first and gmask have room for
+    int* list_count = nullptr;
+    int* item_prob = nullptr;
 };
 
-// One block of CH threads per source chunk: group (kGroup) and chunk boxes of the
-// records with a nonzero charge.  Block 0 also zeroes the item counter for
-// the cull that follows.
-__device__ __forceinline__ void chunk_boxes_body(const PairArgs& A, const CullArgs& C,
-                                                 const int chunk) {
-    __shared__ Box s_g[kGroupsPerChunk];
-    const int n_chunks = A.dyn ? A.dyn[0] : A.n_chunks;
-    if (chunk == 0) {
-        if (threadIdx.x == 0) {
-            if (C.item_count) *C.item_count = 0;
-            if (C.work) *C.work = 0;
-            if (C.done) *C.done = 0;
-        }
-        if (C.hist)
-            for (int b = (int)threadIdx.x; b < kCostBuckets; b += (int)blockDim.x) C.hist[b] = 0;
+// Block 0 of the chunk boxes zeroes the counters of the cull that follows.
+__device__ __forceinline__ void chunk_boxes_reset(const CullArgs& C, const int chunk) {
+    if (chunk != 0) return;
+    if (threadIdx.x == 0) {
+        if (C.item_count) *C.item_count = 0;
+        if (C.work) *C.work = 0;
+        if (C.done) *C.done = 0;
     }
-    if (chunk >= n_chunks) return;
-    const int j = chunk * CH + (int)threadIdx.x;
-    const float4 g0 = A.geo[2 * j], g1 = A.geo[2 * j + 1];
-    const bool valid = A.qq[j].x != 0.f;
-    const int x = (int)(-0.5f * g0.x), y = (int)(-0.5f * g0.z), z = (int)(-0.5f * g1.x);
+    if (C.hist)
+        for (int b = (int)threadIdx.x; b < kCostBuckets; b += (int)blockDim.x) C.hist[b] = 0;
+}
+
+// One block of CH threads per source chunk, thread i with source i's site
+// (valid: a nonzero charge): group (kGroup) and chunk boxes of the valid ones.
+__device__ __forceinline__ void chunk_boxes_reduce(const CullArgs& C, const int chunk,
+                                                   const bool valid, const int x, const int y,
+                                                   const int z) {
+    __shared__ Box s_g[kGroupsPerChunk];
     int xl = valid ? x : 32767, yl = valid ? y : 32767, zl = valid ? z : 32767;
     int xh = valid ? x : -32768, yh = valid ? y : -32768, zh = valid ? z : -32768;
     // min and max over each aligned group of kGroup lanes
@@ -175,6 +181,17 @@ __device__ __forceinline__ void chunk_boxes_body(const PairArgs& A, const CullAr
         }
         C.cbox[chunk] = u;
     }
+}
+
+__device__ __forceinline__ void chunk_boxes_body(const PairArgs& A, const CullArgs& C,
+                                                 const int chunk) {
+    const int n_chunks = A.dyn ? A.dyn[0] : A.n_chunks;
+    chunk_boxes_reset(C, chunk);
+    if (chunk >= n_chunks) return;
+    const int j = chunk * CH + (int)threadIdx.x;
+    const float4 g0 = A.geo[2 * j], g1 = A.geo[2 * j + 1];
+    chunk_boxes_reduce(C, chunk, A.qq[j].x != 0.f, (int)(-0.5f * g0.x), (int)(-0.5f * g0.z),
+                       (int)(-0.5f * g1.x));
 }
 
 // order[] = the items by decreasing cost (a counting sort over the cost
@@ -381,10 +398,8 @@ __device__ __forceinline__ void cull_body(const CullArgs& C, const int tile) {
 // persistent grid and dynamic shared memory pair_smem_bytes(tab_k)
 // (pair_smem_bytes64 for PATH 2).
 //
-// The items come from a problem set PS: one problem (a call of the API, one
-// replica), or the culled replicas of a batch, whose items are numbered one
-// after the other (ProblemList).  PS::count() is the number of items,
-// PS::resolve(g, prob, local) the problem and local item of item g,
+// The items come from a problem set PS, here one problem (a call of the API,
+// one replica).  PS::count() is the number of items, PS::resolve(g, prob, local) the problem and local item of item g,
 // PS::A(prob) / PS::C(prob) that problem's arguments, and PS::first() the
 // arguments whose tables go to shared memory.
 struct OneProblem {
@@ -406,42 +421,16 @@ struct OneProblem {
         local = c.order ? c.order[g] : g;
         return c.items[local];
     }
+    __device__ __forceinline__ int4 mma_item(int g, int& prob) const {
+        prob = 0;
+        return c.items[g];
+    }
     __device__ __forceinline__ const PairArgs& A(int) const { return a; }
     __device__ __forceinline__ const CullArgs& C(int) const { return c; }
     __device__ __forceinline__ const PairArgs& first() const { return a; }
     __device__ __forceinline__ int* work() const { return c.work; }
+    __device__ __forceinline__ int table_entries() const { return c.c2; }
 };
-// The culled replicas list[0 .. n-1] of a batch, their arguments pa[r] and
-// ca[r], and offs[i] the number of items of list[0 .. i-1] (offs[n] = all).
-struct ProblemList {
-    const PairArgs* pa;
-    const CullArgs* ca;
-    const int* list;
-    const int* offs;   // [n + 2]: offs[n + 1] is the next item to take (zeroed with offs)
-    int n;
-    const int* order;  // the items largest first (null: in number order)
-    __device__ __forceinline__ int count() const { return n > 0 ? offs[n] : 0; }
-    __device__ __forceinline__ void resolve(int g, int& prob, int& local) const {
-        if (order) g = order[g];
-        int lo = 0, hi = n;  // the last i with offs[i] <= g
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (offs[mid] <= g) lo = mid;
-            else hi = mid;
-        }
-        prob = list[lo];
-        local = g - offs[lo];
-    }
-    __device__ __forceinline__ int4 item(int g, int& prob, int& local) const {
-        resolve(g, prob, local);
-        return ca[prob].items[local];
-    }
-    __device__ __forceinline__ const PairArgs& A(int p) const { return pa[p]; }
-    __device__ __forceinline__ const CullArgs& C(int p) const { return ca[p]; }
-    __device__ __forceinline__ const PairArgs& first() const { return pa[list[0]]; }
-    __device__ __forceinline__ int* work() const { return const_cast<int*>(offs) + n + 1; }
-};
-
 // The pairs of one staged chunk for one warp: the sources of its live groups
 // (bit g of gmask: group g), in FP32 runs of SUB sources folded into acc64
 // (PATH 0, 1), or term by term in FP64 (PATH 2).  sg/sq: the stage's source
@@ -1045,13 +1034,6 @@ __global__ void __launch_bounds__(NT) pair_kernel_culled(PairArgs A, CullArgs C)
     pair_items_culled<KIND, PATH, NT, RP, SUB, NORM>(OneProblem{A, C});
 }
 
-// The culled replicas of a batch in one persistent launch (point charges,
-// MUFU path): their items are numbered one after the other (ProblemList).
-template <int NT, int RP, int SUB, bool NORM>
-__global__ void __launch_bounds__(NT) pair_kernel_culled_list(ProblemList L) {
-    pair_items_culled<0, 0, NT, RP, SUB, NORM>(L);
-}
-
 // Warp-specialised: NW consumer warps and one producer warp, S stages, at
 // least MINB resident CTAs per SM (a register bound).
 template <int KIND, int PATH, int NW, int RP, int SUB, int S, int MINB, bool NORM = false,
@@ -1062,11 +1044,6 @@ __global__ void __launch_bounds__(NW * 32 + 32, MINB)
     pair_items_culled_ws<KIND, PATH, NW, RP, SUB, NORM, S, PIPE, OneProblem, VOTE>(
         OneProblem{A, C});
 }
-template <int NW, int RP, int SUB, int S, int MINB, bool NORM, bool PIPE = false, int VOTE = 1>
-__global__ void __launch_bounds__(NW * 32 + 32, MINB) pair_kernel_culled_ws_list(ProblemList L) {
-    pair_items_culled_ws<0, 0, NW, RP, SUB, NORM, S, PIPE, ProblemList, VOTE>(L);
-}
-
 // (static: each translation unit that launches them has its own copy)
 static __global__ void __launch_bounds__(CH) chunk_boxes_kernel(PairArgs A, CullArgs C) {
     pdl_wait();
@@ -1078,31 +1055,6 @@ static __global__ void __launch_bounds__(kCullThreads) cull_kernel(CullArgs C) {
     pdl_wait();
     pdl_trigger();
     cull_body(C, (int)blockIdx.x);
-}
-
-static __global__ void __launch_bounds__(1024) order_items_kernel(CullArgs C) {
-    order_items_body(C);
-}
-
-// Sum of one physical target's item partials (its tile's items, in order).
-__device__ __forceinline__ double item_sum(const double* __restrict__ part,
-                                           const int* __restrict__ tile_first,
-                                           const int* __restrict__ tile_items, int tile_size,
-                                           int p) {
-    const int tile = p / tile_size, loc = p - tile * tile_size;
-    const int n = tile_items[tile];
-    const double* q = part + (size_t)tile_first[tile] * tile_size + loc;
-    double s = 0.0;
-    int i = 0;
-    for (; i + 4 <= n; i += 4) {  // four loads in flight, then the adds in order
-        double v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = q[(size_t)(i + u) * tile_size];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) s += v[u];
-    }
-    for (; i < n; ++i) s += q[(size_t)i * tile_size];
-    return s;
 }
 
 }  // namespace lgm

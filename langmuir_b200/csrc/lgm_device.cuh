@@ -129,6 +129,27 @@ __device__ __forceinline__ void fma_if_below(float& acc, float q, float w, unsig
         : "r"(key), "r"(lim), "f"(q), "f"(w));
 }
 
+// The same with w read from shared memory at `addr`, by the lanes that add
+// (the others load nothing and conflict with no one's bank).
+__device__ __forceinline__ void fma_tab_if_below(float& acc, float q, uint32_t addr, unsigned key,
+                                                 unsigned lim) {
+    asm("{\n\t.reg .pred p;\n\t.reg .f32 w;\n\t"
+        "setp.lt.u32 p, %1, %2;\n\t"
+        "@p ld.shared.f32 w, [%4];\n\t"
+        "@p fma.rn.f32 %0, %3, w, %0;\n\t}"
+        : "+f"(acc)
+        : "r"(key), "r"(lim), "f"(q), "r"(addr));
+}
+__device__ __forceinline__ void fma_tab64_if_below(double& acc, double q, uint32_t addr,
+                                                   unsigned key, unsigned lim) {
+    asm("{\n\t.reg .pred p;\n\t.reg .f64 w;\n\t"
+        "setp.lt.u32 p, %1, %2;\n\t"
+        "@p ld.shared.f64 w, [%4];\n\t"
+        "@p fma.rn.f64 %0, %3, w, %0;\n\t}"
+        : "+d"(acc)
+        : "r"(key), "r"(lim), "d"(q), "r"(addr));
+}
+
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
 // Programmatic dependent launch.  A kernel launched with the programmatic

@@ -30,7 +30,7 @@
 #include <vector>
 
 #include "langmuir_b200_kmc.h"
-#include "lgm_cull.cuh"
+#include "lgm_mma.cuh"
 #include "lgm_rng.cuh"
 
 using namespace lgm;
@@ -69,18 +69,10 @@ constexpr int kBalanceTries = 1024;
 
 constexpr int kNT = 128, kRP = 4, kSUB = 32;
 constexpr int kTile = kNT * 2 * kRP;
-constexpr int kCullPerItem = 2;  // source chunks per work item of the culled pair sum
-// The culled pair sum: the warp-specialised kernel (lgm_cull.cuh) with 4
-// target warps of 2 target pairs per thread, a producer warp, 4 stages and 4
-// resident CTAs per SM; items taken largest first (the API's default variant).
-constexpr int kCNW = 4, kCRP = 2, kCStages = 4, kCMinBlocks = 4;
-constexpr int kCSUB = kGroup;  // FP32 runs of the culled sum: one source group
-constexpr int kCVote = 2;      // sources per warp vote of the culled sum (the same bits)
-constexpr int kCThreads = kCNW * 32 + 32;
-constexpr int kCTile = kCNW * 32 * 2 * kCRP;
 // Replicas with room for fewer source chunks than this keep the unculled
-// skip tile: with a handful of chunks the boxes and the cull only add launches.
-constexpr int kCullMinChunks = 8;
+// skip tile.  A standalone replica's step has launches to lose by the boxes
+// and the cull; a batch's has them anyway.
+constexpr int kCullMinChunks = 8, kCullMinChunksBatch = 3;
 
 struct Dev {
     int X, Y, Z, XY, V, hr;
@@ -125,22 +117,24 @@ struct Dev {
     int32_t* bins;             // [ncells + 2]
     int32_t *tkey, *tperm;     // [2 ncap]
     int splits;
-    // Culled pair sums (lgm_cull.cuh; standalone replicas and a batch's
+    // Culled pair sums (lgm_mma.cuh; standalone replicas and a batch's
     // per-phase replicas of point charges): the sources sorted by (charge
     // class, lattice cell) and by site inside a bin (skey: bin per source,
     // stmp: sources scattered by bin, sbins: 3 (ncells + 1) bin counters), the
     // targets scattered by bin before their rank inside it (ttmp, [2 ncap]),
-    // chunk and group boxes, each tile's live chunks and the work items.  A
-    // charge class stays padded to whole chunks.
-    int culled, max_items;
+    // the source fragments and target rows, chunk and group boxes, each
+    // segment's live groups and the work items.  A charge class stays padded
+    // to whole chunks.
+    int culled, segs, per_item, max_items, mask_stride;
     int32_t *skey, *stmp, *sbins, *ttmp;
+    uint32_t* frag;
+    float* q1;
+    uint4* tgt16;
     Box *cbox, *gbox;
-    int32_t* live;
-    int4* items;
-    int32_t *item_count, *tile_first, *tile_items;  // item_count[3]: written, taken, tiles
-                                                    // culled
-    int32_t *chist, *corder;  // item costs' histogram and the largest-first order
-                              // (corder null for a batch's replicas: the batch's)
+    uint8_t* gmask;
+    int4* items;                                    // (a batch's replicas: the batch's list)
+    int32_t *item_count, *tile_first, *tile_items;  // item_count[2]: written, taken
+    int32_t *list_count, *item_prob;                // a batch's list, else null
     int src_cap;   // source records capacity (multiple of CH)
     int tpad_cap;  // per-term target block capacity
     unsigned* err;
@@ -272,19 +266,21 @@ __device__ __forceinline__ void pack_body(const Dev& D, const int j) {
         D.cnt[I_TPAD] = tpad;
     }
     auto record = [&](int dst, int s, float q) {
-        float a = 0.f, b = 0.f, c = 0.f, d = -0.5f;
-        if (s >= 0) {
-            int x, y, z;
-            xyz(D, s, x, y, z);
-            a = -2.f * x; b = -2.f * y; c = -2.f * z;
-            d = (float)(x * x + y * y + z * z) - 0.5f;
-        } else {
-            q = 0.f;
+        int x = 0, y = 0, z = 0;
+        if (s >= 0) xyz(D, s, x, y, z);
+        else q = 0.f;
+        if (D.culled) {
+            store_source(D.frag, D.q1, dst, x, y, z, q);
+            return;
         }
+        const float a = -2.f * x, b = -2.f * y, c = -2.f * z;
+        const float d = (float)(x * x + y * y + z * z) - 0.5f;
         D.geo[2 * dst] = make_float4(a, a, b, b);
         D.geo[2 * dst + 1] = make_float4(c, c, d, d);
         D.qq[dst] = make_float2(q, q);
     };
+    // the group of zero charges that fills a batch of groups (lgm_mma.cuh)
+    if (D.culled && j < kGroup) store_source(D.frag, D.q1, D.src_cap + j, 0, 0, 0, 0.f);
     if (j < nsrc && !D.culled) {  // records past the live chunks are never read
         float q = 0.f;
         int s = -1;
@@ -324,9 +320,13 @@ __device__ __forceinline__ void pack_body(const Dev& D, const int j) {
         for (int term = 0; term < 3; ++term) {
             if (!(D.terms & (1u << term))) continue;
             const int xp = term == 0 ? x : (term == 1 ? -1 - x : 2 * D.X - 1 - x);
-            // padding slots carry w = -1: left out of the cull's boxes, never read
-            D.tgt[(size_t)slot * tpad + j] = make_float4(
-                (float)xp, (float)y, (float)z, j < t ? (float)(xp * xp + y * y + z * z) : -1.f);
+            // padding slots carry a mark (w = -1): left out of the cull's boxes, never read
+            if (D.culled)
+                D.tgt16[(size_t)slot * tpad + j] = target_row(xp, y, z, j >= t);
+            else
+                D.tgt[(size_t)slot * tpad + j] =
+                    make_float4((float)xp, (float)y, (float)z,
+                                j < t ? (float)(xp * xp + y * y + z * z) : -1.f);
             ++slot;
         }
     }
@@ -350,9 +350,9 @@ __device__ __forceinline__ void finalize_body(const Dev& D, const int g) {
             qn[slot] = D.part_norm;
             if (slot < D.nterms) {
                 const int p = slot * tpad + g;
-                const int tile = p / kCTile, loc = p - tile * kCTile;
+                const int tile = p / kSeg, loc = p - tile * kSeg;
                 ni[slot] = D.tile_items[tile];
-                const size_t f = (size_t)D.tile_first[tile] * kCTile + loc;
+                const size_t f = (size_t)D.tile_first[tile] * kSeg + loc;
                 qp[slot] = D.part + f;
                 qn[slot] = D.part_norm + f;
                 nmax = max(nmax, ni[slot]);
@@ -367,8 +367,8 @@ __device__ __forceinline__ void finalize_body(const Dev& D, const int g) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const bool on = i + u < ni[slot];
-                    pv[slot][u] = on ? qp[slot][(size_t)(i + u) * kCTile] : 0.0;
-                    nv[slot][u] = on ? qn[slot][(size_t)(i + u) * kCTile] : 0.f;
+                    pv[slot][u] = on ? qp[slot][(size_t)(i + u) * kSeg] : 0.0;
+                    nv[slot][u] = on ? qn[slot][(size_t)(i + u) * kSeg] : 0.f;
                 }
 #pragma unroll
             for (int slot = 0; slot < 3; ++slot)
@@ -1048,17 +1048,17 @@ __global__ void __launch_bounds__(96) k_finalize_culled(Dev D) {
     double sv = 0.0, sn = 0.0;
     if (g < t && slot < D.nterms) {
         const int p = slot * tpad + g;
-        const int tile = p / kCTile, loc = p - tile * kCTile;
+        const int tile = p / kSeg, loc = p - tile * kSeg;
         const int ni = D.tile_items[tile];
-        const size_t f = (size_t)D.tile_first[tile] * kCTile + loc;
+        const size_t f = (size_t)D.tile_first[tile] * kSeg + loc;
         for (int i = 0; i < ni; i += kRows) {
             double pv[kRows];
             float nv[kRows];
 #pragma unroll
             for (int u = 0; u < kRows; ++u) {
                 const bool on = i + u < ni;
-                pv[u] = on ? D.part[f + (size_t)(i + u) * kCTile] : 0.0;
-                nv[u] = on ? D.part_norm[f + (size_t)(i + u) * kCTile] : 0.f;
+                pv[u] = on ? D.part[f + (size_t)(i + u) * kSeg] : 0.0;
+                nv[u] = on ? D.part_norm[f + (size_t)(i + u) * kSeg] : 0.f;
             }
 #pragma unroll
             for (int u = 0; u < kRows; ++u)
@@ -1094,40 +1094,36 @@ __global__ void __launch_bounds__(1024) k_tbins_scan(Dev D) {
     if (blockIdx.x == 0) block_exclusive_scan(D.bins, D.ncells + 1);
     else block_exclusive_scan(D.sbins, 3 * (D.ncells + 1));
 }
-// Source records and work list of the culled pair sum (lgm_cull.cuh).
+// Source records and work list of the culled pair sum (lgm_mma.cuh).
 __host__ __device__ __forceinline__ PairArgs pair_args(const Dev& D) {
     PairArgs A;
     A.geo = D.geo; A.qq = D.qq; A.splits = D.splits; A.tgt = D.tgt; A.part = D.part;
     A.part_norm = D.part_norm;
     A.c2 = (float)D.cutoff2; A.tab = D.gtab; A.tab_k = D.gauss ? D.gtab_k : 0;
     A.err = D.err; A.dyn = D.cnt + I_NCHUNK;  // dyn[0] = n_chunks, dyn[1] = t_phys
+    A.frag = D.frag; A.q1 = D.q1; A.tgt16 = D.tgt16; A.pad_group = D.src_cap / kGroup;
     return A;
 }
 __host__ __device__ __forceinline__ CullArgs cull_args(const Dev& D) {
     CullArgs C;
     C.cbox = D.cbox; C.gbox = D.gbox;
-    C.tgt = D.tgt; C.dyn = D.cnt + I_NCHUNK;
-    C.c2 = D.cutoff2; C.tile_size = kCTile;
-    C.per_item = kCullPerItem; C.max_items = D.max_items;
-    C.live = D.live; C.live_stride = D.src_cap / CH;
+    C.tgt16 = D.tgt16; C.dyn = D.cnt + I_NCHUNK;
+    C.c2 = D.cutoff2; C.tile_size = kSeg;
+    C.per_item = D.per_item; C.max_items = D.max_items;
+    C.gmask = D.gmask; C.mask_stride = D.mask_stride; C.max_tiles = D.segs;
     C.items = D.items; C.item_count = D.item_count; C.work = D.item_count + 1;
     C.tile_first = D.tile_first; C.tile_items = D.tile_items;
-    // costs from the pair kernel's warp segments; a standalone replica orders
-    // its own items (a batch orders all its culled replicas' items at once)
-    C.warp_targets = 64 * kCRP;
-    C.hist = D.chist;
-    C.order = D.corder;
-    C.done = D.item_count + 2;
+    C.list_count = D.list_count; C.item_prob = D.item_prob;
     return C;
 }
 __global__ void __launch_bounds__(CH) k_chunk_boxes(Dev D) {
     pdl_wait();
     pdl_trigger();
-    chunk_boxes_body(pair_args(D), cull_args(D), (int)blockIdx.x);
+    chunk_boxes_mma_body(pair_args(D), cull_args(D), (int)blockIdx.x);
 }
 __global__ void __launch_bounds__(kCullThreads) k_cull(Dev D) {
     pdl_wait();
-    pdl_trigger(); cull_body(cull_args(D), (int)blockIdx.x); }
+    pdl_trigger(); cull_mma_body(cull_args(D), (int)blockIdx.x, 0); }
 __global__ void k_tscatter(Dev D) {
     pdl_wait();
     pdl_trigger(); tscatter_body(D, LGM_THREAD_INDEX); }
@@ -1196,14 +1192,17 @@ __global__ void __launch_bounds__(1024) kb_tbins_scan(const Dev* R, const int* l
     if (blockIdx.y == 0) block_exclusive_scan(D.bins, D.ncells + 1);
     else if (D.culled) block_exclusive_scan(D.sbins, 3 * (D.ncells + 1));
 }
-// The culled replicas' chunk boxes and tile culls: block b works for replica
-// map[b].x as its chunk or tile map[b].y.
-__global__ void __launch_bounds__(CH) kb_chunk_boxes(const Dev* R, const int2* map) {
+// The culled replicas' chunk boxes and segment culls: block b works for replica
+// map[b].x as its chunk or block of segments map[b].y.  The first block also
+// zeroes the counters of the batch's item list.
+__global__ void __launch_bounds__(CH) kb_chunk_boxes(const Dev* R, const int2* map, int* counts) {
     const Dev& D = R[map[blockIdx.x].x];
-    chunk_boxes_body(pair_args(D), cull_args(D), map[blockIdx.x].y);
+    if (blockIdx.x == 0 && threadIdx.x < 2) counts[threadIdx.x] = 0;
+    chunk_boxes_mma_body(pair_args(D), cull_args(D), map[blockIdx.x].y);
 }
 __global__ void __launch_bounds__(kCullThreads) kb_cull(const Dev* R, const int2* map) {
-    cull_body(cull_args(R[map[blockIdx.x].x]), map[blockIdx.x].y);
+    const int2 m = map[blockIdx.x];
+    cull_mma_body(cull_args(R[m.x]), m.y, m.x);
 }
 // Pairs the work-item kernel tests for the per-phase replicas that do not
 // cull: every physical target against every packed source (one block).
@@ -1213,42 +1212,6 @@ __global__ void kb_tested_pairs(const Dev* R, const int* list, int n, unsigned l
         if (D.culled) continue;
         const int32_t* dyn = D.cnt + I_NCHUNK;
         atomicAdd(out, (unsigned long long)dyn[0] * CH * (unsigned long long)dyn[1]);
-    }
-}
-// One block, after the culls: offs[i] = work items of culled replicas
-// list[0 .. i-1] (i <= n) and offs[n + 1] = 0, the next item to take
-// (ProblemList::work); then order[] = all those items, numbered as
-// ProblemList numbers them, by decreasing cost (the batch's histogram).
-__global__ void __launch_bounds__(1024) kb_item_order(ProblemList L, const Dev* R,
-                                                      const int32_t* hist, int32_t* offs,
-                                                      int32_t* order) {
-    __shared__ int s_off[kCostBuckets];
-    const int n = L.n;
-    for (int i = (int)threadIdx.x; i <= n; i += (int)blockDim.x)
-        offs[i] = i < n ? *R[L.list[i]].item_count : 0;
-    for (int b = (int)threadIdx.x; b < kCostBuckets; b += (int)blockDim.x) s_off[b] = hist[b];
-    __syncthreads();
-    block_exclusive_scan(offs, n + 1);
-    if (threadIdx.x == 0) offs[n + 1] = 0;
-    // the offsets in shared memory for the items' replica searches (up to
-    // kOffsInShared replicas; more search global memory)
-    constexpr int kOffsInShared = 2048;
-    __shared__ int s_offs[kOffsInShared];
-    const bool in_smem = n + 1 <= kOffsInShared;
-    if (in_smem)
-        for (int i = (int)threadIdx.x; i <= n; i += (int)blockDim.x) s_offs[i] = offs[i];
-    cost_offsets(s_off);  // (its barriers also publish s_offs)
-    const int* so = in_smem ? s_offs : offs;
-    const int total = so[n];
-    for (int g = (int)threadIdx.x; g < total; g += (int)blockDim.x) {
-        int lo = 0, hi = n;  // the last replica whose first item is at or before g
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (so[mid] <= g) lo = mid;
-            else hi = mid;
-        }
-        const int c = min(L.C(L.list[lo]).items[g - so[lo]].w, kCostBuckets - 1);
-        order[atomicAdd(&s_off[c], 1)] = g;
     }
 }
 __global__ void __launch_bounds__(kGuardThreadsBatch) kb_guard(const Dev* R, const int4* map) {
@@ -1499,7 +1462,6 @@ struct lgm_kmc {
     int gtab_k = 0;
     int pair_blocks = 0, pair_tiles = 0;
     int cull_grid = 0;  // persistent grid of the culled pair kernel (one wave)
-    int cull_tiles = 0; // target tiles of the culled pair sum (kCTile targets each)
     bool cull_ok = false;  // the culled pair sum's buffers exist
     int sm_count = 0;   // SMs of the device (the guard's grid)
     std::string err;
@@ -1755,15 +1717,22 @@ lgm_status upload_carriers(lgm_kmc* k, const int32_t* e, int ne, const int32_t* 
 using KPairFn = void (*)(PairArgs);
 
 using KCulledFn = void (*)(PairArgs, CullArgs);
-KCulledFn kmc_pair_culled(int gauss) {
-    return gauss ? &pair_kernel_culled_ws<1, 0, kCNW, kCRP, kCSUB, kCStages, kCMinBlocks, true, false, kCVote>
-                 : &pair_kernel_culled_ws<0, 0, kCNW, kCRP, kCSUB, kCStages, kCMinBlocks, true, false, kCVote>;
+KCulledFn kmc_pair_culled(int gauss, int c2) {
+    if (c2 > kMmaTabEntries)
+        return gauss ? &pair_kernel_mma<1, 0, 0, true> : &pair_kernel_mma<0, 0, 0, true>;
+    return gauss ? &pair_kernel_mma<1, 0, kMmaTabGauss, true>
+                 : &pair_kernel_mma<0, 0, kMmaTabPoint, true>;
 }
-size_t kmc_culled_smem(int tab_k) { return ws_smem_bytes(kCStages, tab_k, 4); }
+size_t kmc_culled_smem(int c2, int tab_k) {
+    return mma_smem_bytes(c2 <= kMmaTabEntries ? c2 : tab_k + 1, 4);
+}
 
 // the culled replicas of a batch (point charges), one persistent launch
-constexpr auto kBatchCulled =
-    &pair_kernel_culled_ws_list<kCNW, kCRP, kCSUB, kCStages, kCMinBlocks, true, false, kCVote>;
+using KListFn = void (*)(MmaList);
+KListFn batch_pair_culled(int c2) {
+    return c2 > kMmaTabEntries ? &pair_kernel_mma_list<0, true>
+                               : &pair_kernel_mma_list<kMmaTabPoint, true>;
+}
 
 KPairFn kmc_pair(int gauss, int sorted = 1) {
     if (sorted)
@@ -1815,9 +1784,9 @@ lgm_status enqueue_step(lgm_kmc* k) {
         const PairArgs A = pair_args(D);
         if (D.culled) {
             KCUDA(k, kl(k_chunk_boxes, D.src_cap / CH, CH, 0, st, D));
-            KCUDA(k, kl(k_cull, k->cull_tiles, kCullThreads, 0, st, D));
-            KCUDA(k, kl(kmc_pair_culled(D.gauss), k->cull_grid, kCThreads,
-                        kmc_culled_smem(A.tab_k), st, A, cull_args(D)));
+            KCUDA(k, kl(k_cull, (D.segs + kCullSegs - 1) / kCullSegs, kCullThreads, 0, st, D));
+            KCUDA(k, kl(kmc_pair_culled(D.gauss, D.cutoff2), k->cull_grid, kMmaThreads,
+                        kmc_culled_smem(D.cutoff2, A.tab_k), st, A, cull_args(D)));
         } else {
             KCUDA(k, kl(kmc_pair(D.gauss, D.sorted), dim3(k->pair_tiles, D.splits), kNT,
                         pair_smem_bytes(A.tab_k), st, A));
@@ -2008,16 +1977,17 @@ static lgm_status kmc_create_impl(const lgm_params* pin, int32_t device, uint32_
     DA(D.cnt, I_NUM); DA(D.ctr, C_NUM);
     DA(D.geo, 2 * D.src_cap); DA(D.qq, D.src_cap);
     DA(D.tgt, tphys_cap + kTile);
-    // The pair sum culls source chunks beyond the cutoff when the replica has
-    // room for kCullMinChunks of them: a standalone replica always, a batch's
+    // The pair sum culls sources beyond the cutoff when the replica has room
+    // for enough chunks of them: a standalone replica always, a batch's
     // replica when the batch puts it on the per-phase kernels (partition_batch
     // sets D.culled; its partials then take either layout).
     const int src_chunks = D.src_cap / CH;
-    k->cull_ok = D.coulomb && src_chunks >= kCullMinChunks;
+    k->cull_ok = D.coulomb && src_chunks >= (pool ? kCullMinChunksBatch : kCullMinChunks);
     D.culled = (k->cull_ok && !pool) ? 1 : 0;
-    k->cull_tiles = (tphys_cap + kCTile - 1) / kCTile;
-    D.max_items = std::min(kMaxItemsPerTile, (src_chunks + kCullPerItem - 1) / kCullPerItem);
-    const size_t part_cull = (size_t)k->cull_tiles * D.max_items * kCTile;
+    D.segs = tphys_cap / kSeg;
+    mma_items(D.segs, src_chunks * kGroupsPerChunk, pool != nullptr, &D.per_item, &D.max_items);
+    D.mask_stride = (src_chunks + 31) / 32 * 32;
+    const size_t part_cull = (size_t)D.segs * D.max_items * kSeg;
     const size_t part_n = D.culled ? part_cull
                           : k->cull_ok ? std::max(part_cull, (size_t)D.splits * tphys_cap)
                                        : (size_t)D.splits * tphys_cap;
@@ -2025,11 +1995,12 @@ static lgm_status kmc_create_impl(const lgm_params* pin, int32_t device, uint32_
     if (k->cull_ok) {
         DA(D.skey, D.cap_e + D.cap_h + nd_src); DA(D.stmp, D.cap_e + D.cap_h + nd_src);
         DA(D.ttmp, 2 * ncap);
+        DA(D.frag, (size_t)(D.src_cap + kGroup) * 4); DA(D.q1, D.src_cap + kGroup);
+        DA(D.tgt16, tphys_cap);
         DA(D.cbox, src_chunks); DA(D.gbox, (size_t)src_chunks * kGroupsPerChunk);
-        DA(D.live, (size_t)k->cull_tiles * src_chunks);
-        DA(D.items, (size_t)k->cull_tiles * D.max_items);
-        DA(D.item_count, 3); DA(D.tile_first, k->cull_tiles); DA(D.tile_items, k->cull_tiles);
-        DA(D.chist, kCostBuckets); DA(D.corder, (size_t)k->cull_tiles * D.max_items);
+        DA(D.gmask, (size_t)D.segs * D.mask_stride);
+        if (!pool) DA(D.items, (size_t)D.segs * D.max_items);
+        DA(D.item_count, 2); DA(D.tile_first, D.segs); DA(D.tile_items, D.segs);
     }
     DA(D.Vt, 2 * ncap); DA(D.Nt, 2 * ncap);
     DA(D.err, 1);
@@ -2073,15 +2044,17 @@ static lgm_status kmc_create_impl(const lgm_params* pin, int32_t device, uint32_
         for (int sorted = 0; sorted < 2; ++sorted)
             cudaFuncSetAttribute(kmc_pair(1, sorted), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)pair_smem_bytes(kmax));
-        cudaFuncSetAttribute(kmc_pair_culled(1), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kmc_culled_smem(kmax));
+        cudaFuncSetAttribute(kmc_pair_culled(1, D.cutoff2),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kmc_culled_smem(D.cutoff2, kmax));
     }
     cudaMemcpy(crank_d, crank.data(), sizeof(int32_t) * crank.size(), cudaMemcpyHostToDevice);
     D.cell_rank = crank_d;
     if (D.culled) {
         int cbps = 1;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cbps, kmc_pair_culled(D.gauss), kCThreads,
-                                                      kmc_culled_smem(D.gauss ? D.gtab_k : 0));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &cbps, kmc_pair_culled(D.gauss, D.cutoff2), kMmaThreads,
+            kmc_culled_smem(D.cutoff2, D.gauss ? D.gtab_k : 0));
         k->cull_grid = n_sms * std::max(1, cbps);
     }
     {
@@ -2372,12 +2345,13 @@ struct lgm_kmc_batch {
     int *d_fused = nullptr, *d_classic = nullptr;
     // per-phase replicas whose pair sum culls source chunks (point charges):
     // their chunk boxes, tile culls and one persistent launch over all their
-    // work items (lgm_cull.cuh, ProblemList); the others take the items kernel
+    // work items (lgm_mma.cuh, MmaList); the others take the items kernel
     std::vector<int> culled;
     int* d_culled = nullptr;
-    int32_t* d_coffs = nullptr;      // [culled + 2] work-item offsets, next item taken
-    int32_t* d_chist = nullptr;      // [kCostBuckets] the culled items' costs
-    int32_t* d_corder = nullptr;     // the culled items, largest first
+    int32_t* d_ccount = nullptr;     // [2] items in the list, items claimed
+    int4* d_citems = nullptr;        // the culled replicas' items
+    int32_t* d_cprob = nullptr;      // the replica of each
+    int ctab = 0;                    // the largest cutoff^2 of the culled replicas
     PairArgs* d_cpargs = nullptr;    // [count], filled for the culled replicas
     CullArgs* d_cargs = nullptr;     // [count]
     int2 *map_box = nullptr, *map_cull = nullptr;
@@ -2470,19 +2444,16 @@ lgm_status enqueue_batch_items(lgm_kmc_batch* b, cudaStream_t st) {
     return LGM_OK;
 }
 
-// The batched pair sum: the culled replicas' chunk boxes, tile culls, item
-// offsets and one persistent launch over all their items, then the work-item
-// kernel over the rest.
+// The batched pair sum: the culled replicas' chunk boxes, culls and one
+// persistent launch over all their items, then the work-item kernel over the
+// rest.
 lgm_status enqueue_batch_pair(lgm_kmc_batch* b, cudaStream_t st) {
     if (!b->culled.empty()) {
-        const int n = (int)b->culled.size();
-        kb_chunk_boxes<<<b->nb_box, CH, 0, st>>>(b->d_reps, b->map_box);
+        kb_chunk_boxes<<<b->nb_box, CH, 0, st>>>(b->d_reps, b->map_box, b->d_ccount);
         kb_cull<<<b->nb_cull, kCullThreads, 0, st>>>(b->d_reps, b->map_cull);
-        kb_item_order<<<1, 1024, 0, st>>>(
-            ProblemList{b->d_cpargs, b->d_cargs, b->d_culled, b->d_coffs, n, nullptr}, b->d_reps,
-            b->d_chist, b->d_coffs, b->d_corder);
-        kBatchCulled<<<b->cull_grid, kCThreads, kmc_culled_smem(0), st>>>(
-            ProblemList{b->d_cpargs, b->d_cargs, b->d_culled, b->d_coffs, n, b->d_corder});
+        batch_pair_culled(b->ctab)<<<b->cull_grid, kMmaThreads, kmc_culled_smem(b->ctab, 0), st>>>(
+            MmaList{b->d_cpargs, b->d_cargs, b->d_citems, b->d_cprob, b->d_ccount, b->culled[0],
+                    b->ctab});
     }
     return enqueue_batch_items(b, st);
 }
@@ -2627,36 +2598,37 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
     // culled pair sums for the per-phase replicas with room for enough chunks
     // (point charges: the Gaussian tables differ between replicas)
     b->culled.clear();
-    for (int r = 0; r < (int)b->hD.size(); ++r) {
-        b->hD[r].culled = 0;
-        b->hD[r].chist = b->reps[r]->D.chist;
-        b->hD[r].corder = b->reps[r]->D.corder;
-    }
+    for (Dev& D : b->hD) D.culled = 0;
     for (int r : b->classic)
         if (b->reps[r]->cull_ok && !b->gauss) {
             b->hD[r].culled = 1;
             b->culled.push_back(r);
         }
-    // the culled items' cost histogram and order are the batch's
-    for (int32_t** p : {&b->d_coffs, &b->d_chist, &b->d_corder}) {
+    // the culled replicas' items are one list, the batch's
+    for (void** p : {(void**)&b->d_ccount, (void**)&b->d_citems, (void**)&b->d_cprob}) {
         if (*p) cudaFree(*p);
         *p = nullptr;
     }
-    size_t order_cap = 1;
-    for (int r : b->culled) order_cap += (size_t)b->reps[r]->cull_tiles * b->hD[r].max_items;
-    if (cudaMalloc(&b->d_coffs, sizeof(int32_t) * (b->culled.size() + 2)) != cudaSuccess ||
-        cudaMalloc(&b->d_chist, sizeof(int32_t) * kCostBuckets) != cudaSuccess ||
-        cudaMalloc(&b->d_corder, sizeof(int32_t) * order_cap) != cudaSuccess)
-        return bfail(b, LGM_ERR_CUDA, "work-item offsets");
+    size_t item_cap = 1;
+    b->ctab = 0;
+    for (int r : b->culled) {
+        item_cap += (size_t)b->hD[r].segs * b->hD[r].max_items;
+        b->ctab = std::max(b->ctab, b->hD[r].cutoff2);
+    }
+    if (cudaMalloc(&b->d_ccount, sizeof(int32_t) * 2) != cudaSuccess ||
+        cudaMalloc(&b->d_citems, sizeof(int4) * item_cap) != cudaSuccess ||
+        cudaMalloc(&b->d_cprob, sizeof(int32_t) * item_cap) != cudaSuccess)
+        return bfail(b, LGM_ERR_CUDA, "work items");
     std::vector<int2> box, cull;
     std::vector<PairArgs> cpargs(b->hD.size());
     std::vector<CullArgs> cargs(b->hD.size());
     for (int r : b->culled) {
         Dev& D = b->hD[r];
-        D.chist = b->d_chist;
-        D.corder = nullptr;
+        D.items = b->d_citems;
+        D.item_prob = b->d_cprob;
+        D.list_count = b->d_ccount;
         for (int c = 0; c < D.src_cap / CH; ++c) box.push_back(make_int2(r, c));
-        for (int t = 0; t < b->reps[r]->cull_tiles; ++t) cull.push_back(make_int2(r, t));
+        for (int t = 0; t * kCullSegs < D.segs; ++t) cull.push_back(make_int2(r, t));
         cpargs[r] = pair_args(D);
         cargs[r] = cull_args(D);
     }
@@ -2700,8 +2672,8 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
     if (!b->culled.empty()) {
         int dev_sms = 0, cbps = 1;
         cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, b->device);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cbps, kBatchCulled, kCThreads,
-                                                      kmc_culled_smem(0));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cbps, batch_pair_culled(b->ctab),
+                                                      kMmaThreads, kmc_culled_smem(b->ctab, 0));
         b->cull_grid = std::max(1, dev_sms) * std::max(1, cbps);
     }
     b->nb_guard = (int)guard.size();
@@ -2780,8 +2752,8 @@ lgm_status lgm_kmc_batch_destroy(lgm_kmc_batch* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     void* ptrs[] = {b->d_reps, b->d_pargs, b->d_items, b->map_car, b->map_pack, b->map_fin,
                     b->map_guard, b->map_bins, b->d_fused, b->d_classic, b->d_culled,
-                    b->d_coffs, b->d_cpargs, b->d_cargs, b->map_box, b->map_cull,
-                    b->d_chist, b->d_corder};
+                    b->d_ccount, b->d_cpargs, b->d_cargs, b->map_box, b->map_cull,
+                    b->d_citems, b->d_cprob};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (b->fork) cudaEventDestroy(b->fork);

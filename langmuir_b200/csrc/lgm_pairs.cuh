@@ -64,6 +64,12 @@ struct PairArgs {
     // this is prefactor-free N = sum_j |q_j| w(r_j), the error scale of the
     // target's potential.  Layout [splits][t_phys].
     float* part_norm = nullptr;
+    // Tensor-core sums (lgm_mma.cuh): source fragments (64 words per group of
+    // 16, one zero-charge group at pad_group), charges, target rows
+    const uint32_t* frag = nullptr;
+    const float* q1 = nullptr;        // [n_pad + 16]
+    int pad_group = 0;
+    const uint4* tgt16 = nullptr;     // [t_phys], rounded up to whole segments
 };
 
 // Kernel launched with dynamic shared memory pair_smem_bytes(tab_k).
