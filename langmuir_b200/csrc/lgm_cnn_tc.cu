@@ -330,6 +330,8 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
 
 }  // namespace
 
+unsigned lgm_cnn_net_error_take();  // lgm_cnn_net.cu
+
 extern "C" {
 
 lgm_status lgm_cnn_conv3x3_fwd_tc(const void* x, const void* w, const float* bias, void* act,
@@ -396,6 +398,9 @@ lgm_status lgm_cnn_error(uint32_t* flags) {
     if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof v) != cudaSuccess ||
         cudaMemcpyToSymbol(g_tc_error, &zero, sizeof zero) != cudaSuccess)
         return LGM_ERR_CUDA;
+    const unsigned net = lgm_cnn_net_error_take();
+    if (net == ~0u) return LGM_ERR_CUDA;
+    v |= net;
     *flags = v;
     return v ? LGM_ERR_TIMEOUT : LGM_OK;
 }

@@ -54,6 +54,9 @@ N.SIGNATURES.update({
     "lgm_cnn_to_bf16": (_i32, [_vp, _vp, _i32, _vp, _vp]),
     "lgm_cnn_conv3x3_fwd_tc": (_i32, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
     "lgm_cnn_error": (_i32, [ctypes.POINTER(ctypes.c_uint32)]),
+    "lgm_cnn_net_bytes": (ctypes.c_size_t, [_i32, _i32, _i32, _i32]),
+    "lgm_cnn_net_forward": (_i32, [_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp]),
+    "lgm_cnn_net_backward": (_i32, [_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp]),
 })
 _CNN_SYMBOLS = [k for k in N.SIGNATURES if k.startswith("lgm_cnn_")]
 if N._lib is not None:
@@ -183,62 +186,38 @@ def check_image_shape(H, W):
         raise ValueError(f"image {H}x{W}: the kernels need H % 64 == 0 and W % 128 == 0")
 
 
+def _masters(params):
+    """The twelve FP32 masters as contiguous tensors and a C array of their pointers."""
+    ps = [p if p.dtype == torch.float32 and p.is_contiguous() else p.float().contiguous()
+          for p in params]
+    return ps, (_vp * len(ps))(*[p.data_ptr() for p in ps])
+
+
 def network_forward(x16, params, keep=True):
     """x16: [B,H,W,1] bf16; params: FP32 masters in PARAM_SHAPES order.
-    Returns y [B,2] fp32 and (keep) the tensors the backward pass reads."""
-    c1w, c1b, c2w, c2b, c3w, c3b, c4w, c4b, f1w, f1b, f2w, f2b = params
+    Returns y [B,2] fp32 and (keep) what the backward pass reads."""
     B, H, W, _ = x16.shape
     check_image_shape(H, W)
-    w1 = conv_weights_bf16(c1w, 1)
-    w2, w3, w4 = (conv_weights_bf16(w, CH) for w in (c2w, c3w, c4w))
-    a1, p1 = conv3x3(x16, w1, c1b, H, W, keep_act=keep)
-    a2, p2 = conv3x3(p1, w2, c2b, H // 2, W // 2, keep_act=keep)
-    a3, p3 = conv3x3(p2, w3, c3b, H // 4, W // 4, keep_act=keep)
-    a4, _ = conv3x3(p3, w4, c4b, H // 8, W // 8, keep_act=True, pool=False)
-    g32, g16 = gap_fwd(a4)
-    f1w16, f2w16 = f1w.to(torch.bfloat16), f2w.to(torch.bfloat16)
-    # h = relu(g W1^T + b1): A(b, c) = g16[b][c], B(c, j) = W1[j][c]
-    h32 = gemm(g16, CH, 1, f1w16, 1, CH, B, HIDDEN, CH, bias=f1b, relu=True)
-    h16 = to_bf16(h32)
-    y = gemm(h16, HIDDEN, 1, f2w16, 1, HIDDEN, B, OUTPUTS, HIDDEN, bias=f2b)
-    saved = (x16, w2, w3, w4, f1w16, f2w16, a1, p1, a2, p2, a3, p3, a4, g16, h32, h16) if keep else None
-    return y, saved
+    x16 = x16.contiguous()
+    masters, ptrs = _masters(params)
+    work = torch.empty(N.lib().lgm_cnn_net_bytes(B, H, W, int(keep)), dtype=torch.uint8,
+                       device=x16.device)
+    y = torch.empty(B, OUTPUTS, dtype=torch.float32, device=x16.device)
+    _ok(N.lib().lgm_cnn_net_forward(_p(x16), ptrs, _p(work), _p(y), B, H, W, int(keep), _stream()))
+    return y, ((x16, work) if keep else None)
 
 
 def network_backward(dy, saved):
     """Gradients of the FP32 masters (PARAM_SHAPES order) from dL/dy."""
-    x16, w2, w3, w4, f1w16, f2w16, a1, p1, a2, p2, a3, p3, a4, g16, h32, h16 = saved
+    x16, kept = saved
     B, H, W, _ = x16.shape
-    dev = dy.device
-    dy16 = to_bf16(dy.contiguous())
-    ones = torch.ones(B, dtype=torch.bfloat16, device=dev)
-    z = lambda *s: torch.zeros(*s, dtype=torch.float32, device=dev)
-    # head: dW2 = dy^T h, db2 = 1^T dy, dh = dy W2 (masked by h > 0)
-    df2w = gemm(dy16, 1, OUTPUTS, h16, HIDDEN, 1, OUTPUTS, HIDDEN, B, out=z(OUTPUTS, HIDDEN))
-    df2b = gemm(ones, 0, 1, dy16, OUTPUTS, 1, 1, OUTPUTS, B, out=z(1, OUTPUTS)).view(OUTPUTS)
-    dh = gemm(dy16, OUTPUTS, 1, f2w16, HIDDEN, 1, B, HIDDEN, OUTPUTS)
-    dh16 = to_bf16(dh, relu_mask=h32)
-    df1w = gemm(dh16, 1, HIDDEN, g16, CH, 1, HIDDEN, CH, B, out=z(HIDDEN, CH))
-    df1b = gemm(ones, 0, 1, dh16, HIDDEN, 1, 1, HIDDEN, B, out=z(1, HIDDEN)).view(HIDDEN)
-    dg = gemm(dh16, HIDDEN, 1, f1w16, CH, 1, B, CH, HIDDEN)
-    # conv stack
-    dA4 = gap_relu_bwd(a4, dg)
-    dc4w, dc4b = z(CH, 9 * CH), z(CH)
-    conv3x3_wgrad(p3, dA4, dc4w, dc4b, H // 8, W // 8)
-    dp3 = conv3x3_dgrad(dA4, w4, H // 8, W // 8)
-    dA3 = relu_pool_bwd(a3, dp3, True)
-    dc3w, dc3b = z(CH, 9 * CH), z(CH)
-    conv3x3_wgrad(p2, dA3, dc3w, dc3b, H // 4, W // 4)
-    dp2 = conv3x3_dgrad(dA3, w3, H // 4, W // 4)
-    dA2 = relu_pool_bwd(a2, dp2, True)
-    dc2w, dc2b = z(CH, 9 * CH), z(CH)
-    conv3x3_wgrad(p1, dA2, dc2w, dc2b, H // 2, W // 2)
-    dp1 = conv3x3_dgrad(dA2, w2, H // 2, W // 2)
-    dA1 = relu_pool_bwd(a1, dp1, True)
-    dc1w16, dc1b = z(CH, 16), z(CH)
-    conv3x3_wgrad(x16, dA1, dc1w16, dc1b, H, W)
-    dc1w = dc1w16[:, :9].contiguous()
-    return (dc1w, dc1b, dc2w, dc2b, dc3w, dc3b, dc4w, dc4b, df1w, df1b, df2w, df2b)
+    dy = dy.contiguous()
+    grads = [torch.empty(shape, dtype=torch.float32, device=dy.device) for _, shape in PARAM_SHAPES]
+    work = torch.empty(N.lib().lgm_cnn_net_bytes(B, H, W, 2), dtype=torch.uint8, device=dy.device)
+    gptrs = (_vp * len(grads))(*[g.data_ptr() for g in grads])
+    _ok(N.lib().lgm_cnn_net_backward(_p(x16), _p(kept), _p(dy), _p(work), gptrs, B, H, W,
+                                     _stream()))
+    return tuple(grads)
 
 
 class SurrogateFn(torch.autograd.Function):
