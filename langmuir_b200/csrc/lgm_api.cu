@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -17,6 +18,7 @@
 #include "lgm_context.hpp"
 #include "lgm_cull.cuh"
 #include "lgm_mma.cuh"
+#include "lgm_small.cuh"
 
 using namespace lgm;
 
@@ -25,6 +27,11 @@ namespace {
 thread_local std::string g_create_error;
 
 constexpr int kMaxSplits = 64;
+// The host-buffer call of few sources: bytes its CTAs may read over the bus (a
+// copy to the device costs about 5 us), and polls of the kernel's word before
+// the stream is waited for (a few milliseconds).
+constexpr size_t kZeroCopyBytes = 96 * 1024;
+constexpr int kFlagPolls = 1 << 20;
 constexpr int kDrainIds = 35;       // Grid::m_specialAgentReserve (cubicgrid.cpp:22)
 
 lgm_status fail(lgm_ctx* c, lgm_status st, const std::string& msg) {
@@ -831,6 +838,88 @@ int choose_variant(const lgm_ctx* c, int kind, const Shape& sh) {
     return v;
 }
 
+// Entries of the table a one-kernel call holds in shared memory.
+int small_table(const lgm_ctx* c, int kind) {
+    if (c->cfg.path == LGM_PATH_TABLE64) return c->rtab_k + 1;
+    if (c->cfg.path == LGM_PATH_TABLE) return (kind == LGM_GAUSS ? c->gtab_k : c->rtab_k) + 1;
+    return kind == LGM_GAUSS ? c->gtab_k + 1 : 0;
+}
+
+using SmallFn = void (*)(SmallArgs);
+SmallFn small_fn(int kind, int path) {
+    if (path == LGM_PATH_TABLE64) return &small_sums<0, 2>;
+    if (path == LGM_PATH_TABLE) return &small_sums<0, 1>;
+    return kind == LGM_GAUSS ? &small_sums<1, 0> : &small_sums<0, 0>;
+}
+
+// A call of few sources takes the one-kernel form (lgm_small.cuh): up to
+// kSmallSources of them and kSmallPairs unculled pairs, where the chain's
+// launches cost more than the pairs it culls, with the FP32C precision, no
+// variant forced or tuned for the size, no pair counting, and a table that
+// leaves two CTAs their shared memory.
+bool small_call(const lgm_ctx* c, int kind, const Shape& sh, int n, int t) {
+    if (c->cfg.precision == LGM_PREC_FP64 || c->forced_variant >= 0 || c->counting) return false;
+    if (n < 1 || n > kSmallSources || (long long)n * t * sh.nterms > kSmallPairs) return false;
+    if (c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks))) return false;
+    return small_smem(n, small_table(c, kind), c->cfg.path == LGM_PATH_TABLE64 ? 8 : 4) <= kSmallSmem;
+}
+
+// flag: null, or the host-visible word the last CTA writes {call, error} to.
+lgm_status launch_small(lgm_ctx* c, int kind, unsigned terms, const int32_t* src, const int32_t* q,
+                        int n, const int32_t* tgt, int t, int all_sites, double* out,
+                        cudaStream_t st, unsigned long long* flag, unsigned call) {
+    const lgm_config& cf = c->cfg;
+    SmallArgs S{};
+    S.src = src; S.q = q; S.n = n;
+    S.tgt = all_sites ? nullptr : tgt; S.t = t;
+    S.X = cf.grid_x; S.Y = cf.grid_y; S.XY = c->xy; S.volume = c->volume; S.drains = kDrainIds;
+    S.shift = c->cell_shift; S.cells_x = c->cells_x; S.cells_y = c->cells_y; S.ncells = c->ncells;
+    S.cell_rank = c->d_cell_rank;
+    S.terms = terms;
+    S.c2 = (float)(cf.electrostatic_cutoff * cf.electrostatic_cutoff);
+    if (cf.path == LGM_PATH_TABLE64) S.tab64 = kind == LGM_GAUSS ? c->d_gtab64 : c->d_rtab64;
+    else if (cf.path == LGM_PATH_TABLE) S.tab = kind == LGM_GAUSS ? c->d_gtab : c->d_rtab;
+    else S.tab = c->d_gtab;
+    S.tab_k = small_table(c, kind) - 1;
+    S.prefactor = cf.electrostatic_prefactor;
+    S.out = out;
+    S.err = c->d_err;
+    S.done = reinterpret_cast<unsigned*>(c->d_item_count + 3);
+    S.flag = flag;
+    S.call = call;
+    // few segments: a CTA's warps share one, each with a slice of the groups
+    const int segs = (t + kSeg - 1) / kSeg, batches = (n + 4 * kGroup - 1) / (4 * kGroup);
+    S.split = kSmallWarps;
+    while (S.split > 1 && (S.split > batches || segs * S.split > 2 * kSmallWarps * c->sm_count))
+        S.split /= 2;
+    const int per = kSmallWarps / S.split;
+    const int grid = std::min((segs + per - 1) / per, 4 * c->sm_count);
+    if (c->timing) LGM_CUDA(c, cudaEventRecord(c->ev_pair0, st));
+    LGM_CUDA(c, launch_chain(c->overlap, small_fn(kind, cf.path), grid, kSmallThreads,
+                             small_smem(n, S.tab_k + 1, cf.path == LGM_PATH_TABLE64 ? 8 : 4), st, S));
+    if (c->timing) {
+        LGM_CUDA(c, cudaEventRecord(c->ev_pair1, st));
+        c->timed_pending = true;
+    }
+    c->last.ctas = grid;
+    c->last.threads = kSmallThreads;
+    c->last.targets_per_thread = 1;
+    c->last.variant = kDefaultVariant;
+    c->last.kernel_launches = 1;
+    c->last.pairs_tested = (int64_t)popcount3(terms) * t * (int64_t)n;
+    c->last.splits = 0;
+    return LGM_OK;
+}
+
+void reset_last(lgm_ctx* c) {
+    c->last = lgm_launch_info{};
+    c->last.pair_kernel_ms = -1.f;
+    c->last.variant = -1;
+    c->last.pairs_examined = -1;
+    c->timed_pending = false;
+    c->count_pending = false;
+}
+
 // Shared launch sequence.  d_src/d_q: n sources; d_tgt_site: t targets (or
 // all lattice sites when all_sites).  Everything on `st`.
 lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t* d_src,
@@ -838,12 +927,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
                              int all_sites, double* d_out, cudaStream_t st,
                              unsigned* err_out = nullptr) {
     const lgm_config& cf = c->cfg;
-    c->last = lgm_launch_info{};
-    c->last.pair_kernel_ms = -1.f;
-    c->last.variant = -1;
-    c->last.pairs_examined = -1;
-    c->timed_pending = false;
-    c->count_pending = false;
+    reset_last(c);
     if (t == 0) return LGM_OK;
     if (n == 0) {
         LGM_CUDA(c, launch_chain(c->overlap, fill_zero, (t + 255) / 256, 256, 0, st, d_out, t,
@@ -852,6 +936,10 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         return LGM_OK;
     }
     const Shape sh = shape_of(n, t, terms);
+    // (err_out: the host-buffer call, which takes the small form itself)
+    if (!err_out && small_call(c, kind, sh, n, t))
+        return launch_small(c, kind, terms, d_src, d_q, n, d_tgt_site, t, all_sites, d_out, st, nullptr,
+                            0);
     const int v = choose_variant(c, kind, sh);
     const int fmt =
         cf.precision == LGM_PREC_FP64 || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
@@ -1158,9 +1246,11 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
         if ((e = cudaMalloc(&c->d_cell_rank, sizeof(int32_t) * rank.size())) != cudaSuccess ||
             (e = cudaMalloc(&c->d_bins, sizeof(int32_t) * (2 * c->bins_stride + 4))) !=
                 cudaSuccess ||
-            (e = cudaMalloc(&c->d_item_count, 3 * sizeof(int32_t))) != cudaSuccess ||
+            (e = cudaMalloc(&c->d_item_count, 4 * sizeof(int32_t))) != cudaSuccess ||
             (e = cudaMalloc(&c->d_cost_hist, kCostBuckets * sizeof(int32_t))) != cudaSuccess)
             return bail("cudaMalloc", e);
+        if ((e = cudaMemset(c->d_item_count, 0, 4 * sizeof(int32_t))) != cudaSuccess)
+            return bail("cudaMemset", e);
         // the source bins follow the target bins, 16-byte aligned (the scan reads int4)
         c->d_sbins = c->d_bins + c->bins_stride;
         if ((e = cudaMemcpy(c->d_cell_rank, rank.data(), sizeof(int32_t) * rank.size(),
@@ -1198,6 +1288,10 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
                 c->bps[v][fi] = bps;
             }
     }
+    for (int k : {LGM_POINT, LGM_GAUSS})
+        if ((e = cudaFuncSetAttribute(small_fn(k, cf.path), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSmallSmem)) != cudaSuccess)
+            return bail("cudaFuncSetAttribute", e);
     *out = c;
     return LGM_OK;
 }
@@ -1404,6 +1498,8 @@ lgm_status lgm_potentials(lgm_ctx* c, lgm_kind kind, uint32_t terms, const int32
     if ((s = grow_host(c, &c->h_o, &c->ho_cap, (size_t)t + 1)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_t, &c->t_cap, words)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_o, &c->o_cap, (size_t)t + 1)) != LGM_OK) return s;
+    const Shape sh = shape_of(n, t, terms);
+    const bool small = n > 0 && small_call(c, kind, sh, n, t);
     // The sites are checked on the device (prep_records), which gives each an
     // empty record and raises an error bit; only then are they checked here,
     // for the first bad one (sources first, then targets, as check_sites
@@ -1412,17 +1508,46 @@ lgm_status lgm_potentials(lgm_ctx* c, lgm_kind kind, uint32_t terms, const int32
     std::memcpy(c->h_t, tgt_site, sizeof(int32_t) * t);
     if (n > 0) std::memcpy(c->h_t + t, src_q, sizeof(int32_t) * n);
     if (!alias && n > 0) std::memcpy(c->h_t + t + n, src_site, sizeof(int32_t) * n);
-    LGM_CUDA(c, cudaMemcpyAsync(c->d_t, c->h_t, sizeof(int32_t) * words, cudaMemcpyHostToDevice,
-                                st));
-    const int32_t* d_src = alias ? c->d_t : c->d_t + t + n;
-    unsigned* d_err_out = reinterpret_cast<unsigned*>(c->d_o + t);
-    if ((s = launch_potentials(c, kind, terms, d_src, c->d_t + t, n, c->d_t, t, 0, c->d_o, st,
-                               d_err_out)) != LGM_OK)
-        return s;
-    LGM_CUDA(c, cudaMemcpyAsync(c->h_o, c->d_o, sizeof(double) * ((size_t)t + 1),
-                                cudaMemcpyDeviceToHost, st));
-    LGM_CUDA(c, cudaStreamSynchronize(st));
-    const unsigned e = *reinterpret_cast<const unsigned*>(c->h_o + t);
+    unsigned e = 0;
+    if (small) {
+        // One kernel, results straight into the pinned buffer.  Every CTA reads
+        // the sources: from the pinned staging while that is little, else from
+        // the device after one copy.
+        const size_t reads = sizeof(int32_t) * ((size_t)2 * n * std::min((t + kSeg - 1) / kSeg,
+                                                                         4 * c->sm_count) + t);
+        const int32_t* in = c->h_t;
+        if (reads > kZeroCopyBytes) {
+            LGM_CUDA(c, cudaMemcpyAsync(c->d_t, c->h_t, sizeof(int32_t) * words,
+                                        cudaMemcpyHostToDevice, st));
+            in = c->d_t;
+        }
+        reset_last(c);
+        volatile unsigned long long* flag = reinterpret_cast<volatile unsigned long long*>(c->h_o + t);
+        const unsigned call = ++c->call_number;
+        *flag = (unsigned long long)(call - 1) << 32;
+        if ((s = launch_small(c, kind, terms, alias ? in : in + t + n, in + t, n, in, t, 0, c->h_o, st,
+                              const_cast<unsigned long long*>(flag), call)) != LGM_OK)
+            return s;
+        // the kernel's own word comes sooner than the stream's; if it does not
+        // come soon, wait for the stream (and learn of an error)
+        bool seen = false;
+        for (int i = 0; i < kFlagPolls && !seen; ++i) seen = (unsigned)(*flag >> 32) == call;
+        if (!seen) LGM_CUDA(c, cudaStreamSynchronize(st));
+        std::atomic_thread_fence(std::memory_order_acquire);
+        e = (unsigned)*flag;
+    } else {
+        LGM_CUDA(c, cudaMemcpyAsync(c->d_t, c->h_t, sizeof(int32_t) * words, cudaMemcpyHostToDevice,
+                                    st));
+        const int32_t* d_src = alias ? c->d_t : c->d_t + t + n;
+        unsigned* d_err_out = reinterpret_cast<unsigned*>(c->d_o + t);
+        if ((s = launch_potentials(c, kind, terms, d_src, c->d_t + t, n, c->d_t, t, 0, c->d_o, st,
+                                   d_err_out)) != LGM_OK)
+            return s;
+        LGM_CUDA(c, cudaMemcpyAsync(c->h_o, c->d_o, sizeof(double) * ((size_t)t + 1),
+                                    cudaMemcpyDeviceToHost, st));
+        LGM_CUDA(c, cudaStreamSynchronize(st));
+        e = *reinterpret_cast<const unsigned*>(c->h_o + t);
+    }
     if (e != 0) {
         const lgm_status ds = device_error_status(c, st, e);  // clears the device word
         if (e & (DEVERR_SOURCE_RANGE | DEVERR_TARGET_RANGE)) {

@@ -23,8 +23,13 @@ def fp32_tile(ctx):
 
 def run_all(lgm, dims, cutoff, src, q, tgt, kind, terms, sigma=0.0, path=0):
     with lgm.Coulomb(*dims, cutoff=cutoff, sigma=sigma, path=path) as ctx:
+        auto = ctx.potentials(src, q, tgt, kind, terms)
+        info = ctx.last_launch()
+        assert info["variant"] == len(ctx.variants()) - 1
+        assert info["kernel_launches"] == (1 if len(src) <= 1300 else 7)
+        ctx.set_variant(len(ctx.variants()) - 1)  # the chain, however few the sources
         got = ctx.potentials(src, q, tgt, kind, terms)
-        assert ctx.last_launch()["variant"] == len(ctx.variants()) - 1
+        assert ctx.last_launch()["kernel_launches"] == 7
         ctx.set_variant(fp32_tile(ctx))
         tile = ctx.potentials(src, q, tgt, kind, terms)
     with lgm.Coulomb(*dims, cutoff=cutoff, sigma=sigma, precision=lgm.PREC_FP64) as ctx:
@@ -32,6 +37,8 @@ def run_all(lgm, dims, cutoff, src, q, tgt, kind, terms, sigma=0.0, path=0):
         norm = sum(abs(ctx.potentials(src, np.abs(q), tgt, kind, t)
                        - (0 if t == 1 else ctx.potentials(src, np.abs(q), tgt, kind, 1)))
                    for t in (1, 3, 5) if (t & terms) == t)
+    # the same FP32 runs; only the FP64 order of the item partials differs
+    assert np.all(np.abs(auto - got)[norm > 0] <= 1e-13 * norm[norm > 0])
     return got, tile, exact, norm
 
 
@@ -72,3 +79,42 @@ def test_tile_and_chunk_edges(lgm, n, t, kind, path):
     got, tile, exact, norm = run_all(lgm, dims, 20, src, q, tgt, kind, 3, sigma=1.2, path=path)
     check(got[:-2], tile[:-2], exact[:-2], norm[:-2], TOL64 if path == 2 else TOL32)
     np.testing.assert_allclose(got[-2:], tile[-2:], rtol=1e-12, atol=1e-15)
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 256, 257, 700, 2048, 2049])
+@pytest.mark.parametrize("path", [0, 1, 2])
+def test_one_kernel_call_at_its_edges(lgm, n, path):
+    """Calls around the sizes of the one-kernel form (its sort's powers of two,
+    its largest source count): host buffers, device buffers, every site, sources
+    on one site, repeated calls, against the chain."""
+    import torch
+    dims = (30, 26, 7)
+    V = 30 * 26 * 7
+    rng = np.random.default_rng(n)
+    src = rng.integers(0, V, n).astype(np.int32)  # several charges on a site: legal
+    q = rng.integers(-3, 4, n).astype(np.int32)
+    tgt = rng.integers(0, V, 77).astype(np.int32)
+    with lgm.Coulomb(*dims, cutoff=17, path=path) as ctx:
+        few = ctx.potentials(src, q, tgt, terms=7)
+        assert (ctx.last_launch()["kernel_launches"] == 1) == (n <= 2048)
+        for _ in range(3):
+            np.testing.assert_array_equal(ctx.potentials(src, q, tgt, terms=7), few)
+        site = ctx.kernel1(src, q)
+        d = [torch.as_tensor(a).cuda() for a in (src, q, tgt)]
+        out = torch.zeros(len(tgt), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.potentials_async(d[0].data_ptr(), d[1].data_ptr(), n, d[2].data_ptr(), len(tgt),
+                             out.data_ptr(), terms=7)
+        ctx.sync()
+        np.testing.assert_array_equal(out.cpu().numpy(), few)
+        with pytest.raises(lgm.LgmError, match="source 0"):
+            ctx.potentials(np.where(np.arange(n) == 0, V, src), q, tgt)
+        with pytest.raises(lgm.LgmError, match="target 5"):
+            ctx.potentials(src, q, np.where(np.arange(77) == 5, V + 35, tgt))
+        ctx.set_variant(len(ctx.variants()) - 1)
+        chain = ctx.potentials(src, q, tgt, terms=7)
+        chain_site = ctx.kernel1(src, q)
+        norm = ctx.potentials(src, np.abs(q), tgt) * 3 + 1e-300
+        norm1 = ctx.kernel1(src, np.abs(q)) + 1e-300
+    assert np.all(np.abs(few - chain) <= 1e-13 * norm)
+    assert np.all(np.abs(site - chain_site) <= 1e-13 * norm1)
