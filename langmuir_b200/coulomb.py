@@ -11,21 +11,49 @@ errors raised instead of qFatal.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 
 from . import _native as N
 
 
+_I32, _F64 = np.dtype(np.int32), np.dtype(np.float64)
+
+
 def _i32(a) -> np.ndarray:
+    if type(a) is np.ndarray and a.dtype == _I32 and a.ndim == 1 and a.flags.c_contiguous:
+        return a  # a stepping caller's own array: nothing to convert
     return np.ascontiguousarray(np.asarray(a, dtype=np.int32).ravel())
+
+
+def _ptr(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
+
+
+@functools.cache
+def _call(name: str, *args):
+    """A library function taking addresses.  The arrays' type and layout are
+    checked here (_i32, _out); ndpointer arguments would check them again, about
+    1.5 us each."""
+    return ctypes.CFUNCTYPE(ctypes.c_int32, *args)((name, N.lib()))
+
+
+def _potentials():
+    v, i = ctypes.c_void_p, ctypes.c_int32
+    return _call("lgm_potentials", v, i, ctypes.c_uint32, v, v, i, v, i, v)
+
+
+def _kernel2():
+    v, i = ctypes.c_void_p, ctypes.c_int32
+    return _call("lgm_coulomb_kernel2", v, i, v, v, i, i, v)
 
 
 def _out(out, n: int) -> np.ndarray:
     """A caller's output array (float64, C-contiguous, n long), or a new one."""
     if out is None:
         return np.empty(n, dtype=np.float64)
-    if (not isinstance(out, np.ndarray) or out.dtype != np.float64 or out.shape != (n,)
+    if (not isinstance(out, np.ndarray) or out.dtype != _F64 or out.shape != (n,)
             or not out.flags.c_contiguous):
         raise ValueError(f"out must be a C-contiguous float64 array of length {n}")
     return out
@@ -84,14 +112,16 @@ class Coulomb:
         if len(s) != len(q):
             raise ValueError("src_site and src_q differ in length")
         out = _out(out, len(t))
-        self._check(N.lib().lgm_potentials(self._h, int(kind), int(terms), s, q, len(s), t,
-                                           len(t), out))
+        self._check(_potentials()(self._h, int(kind), int(terms), _ptr(s), _ptr(q), len(s), _ptr(t),
+                                  len(t), _ptr(out)))
         return out
 
     def kernel2(self, s, q, n, kind=N.POINT, out=None):
         s, q = _i32(s), _i32(q)
         out = _out(out, len(s))
-        self._check(N.lib().lgm_coulomb_kernel2(self._h, int(kind), s, q, int(n), len(s), out))
+        if len(q) < int(n):
+            raise ValueError("q has fewer than n entries")
+        self._check(_kernel2()(self._h, int(kind), _ptr(s), _ptr(q), int(n), len(s), _ptr(out)))
         return out
 
     def kernel1(self, s, q, kind=N.POINT):
