@@ -119,8 +119,6 @@ class Coulomb:
     def kernel2(self, s, q, n, kind=N.POINT, out=None):
         s, q = _i32(s), _i32(q)
         out = _out(out, len(s))
-        if len(q) < int(n):
-            raise ValueError("q has fewer than n entries")
         self._check(_kernel2()(self._h, int(kind), _ptr(s), _ptr(q), int(n), len(s), _ptr(out)))
         return out
 
