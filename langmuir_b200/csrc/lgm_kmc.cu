@@ -943,6 +943,39 @@ __device__ void block_try_inject(const Dev& D, InjectState& S, int s, uint32_t s
     __syncthreads();
 }
 
+// The four electrode sources without source.metropolis: their draws and sites
+// do not depend on one another, so lanes 0-3 look them up side by side (one
+// round trip to memory instead of four); lane 0 then injects in order.  A site
+// taken by an earlier source of the step is no longer empty (the two
+// electrodes' faces meet when the lattice is one site wide).
+__device__ __forceinline__ void inject_by_rate(const Dev& D, InjectState& S, uint32_t step) {
+    const int s = threadIdx.x & 3;
+    const Philox4 r = draw(D, step, 0u, RNG_SOURCE + (uint32_t)s);
+    const int idx = (int)uint_below(r.w[0], (uint32_t)(D.Y * D.Z));
+    const int site = D.X * idx + (s % 2 == 0 ? 0 : D.X - 1);
+    const bool yes = D.rate_src[s] > 0 && (s < 2 ? D.et : D.ht)[site] == T_EMPTY &&
+                     D.rate_src[s] > unit_double(r.w[1], r.w[2]);
+    const unsigned all = __ballot_sync(0xffffffffu, yes);
+    int sites[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sites[k] = __shfl_sync(0xffffffffu, site, k);
+    if (threadIdx.x != 0) return;
+    bool in[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const bool e = k < 2;
+        D.ctr[2 * k] += 1;  // attempts (sourceagent.cpp:94)
+        in[k] = ((all >> k) & 1u) && (e ? S.ne < D.cap_e : S.nh < D.cap_h) &&
+                !((k & 1) && in[k & 2] && sites[k & 2] == sites[k]);
+        if (in[k]) {
+            D.ctr[2 * k + 1] += 1;
+            (e ? D.et : D.ht)[sites[k]] = e ? T_ELECTRON : T_HOLE;
+            if (e) D.e_site[S.ne++] = sites[k];
+            else D.h_site[S.nh++] = sites[k];
+        }
+    }
+}
+
 __device__ __forceinline__ void compact_inject_body(const Dev& D, int* warp_sums, double* red) {
     __shared__ InjectState S;
     int ne = D.cnt[I_NE0], nh = D.cnt[I_NH0];
@@ -1012,7 +1045,11 @@ __device__ __forceinline__ void compact_inject_body(const Dev& D, int* warp_sums
         }
     } else {
         // the electrode sources in the reference's order (simulation.cpp:246-249)
-        for (int s = 0; s < 4; ++s) block_try_inject(D, S, s, step, 0u, RNG_SOURCE + (uint32_t)s, red);
+        if (D.src_metro)
+            for (int s = 0; s < 4; ++s)
+                block_try_inject(D, S, s, step, 0u, RNG_SOURCE + (uint32_t)s, red);
+        else if (threadIdx.x < 32)
+            inject_by_rate(D, S, step);
     }
     if (threadIdx.x == 0) {
         D.cnt[I_NE] = S.ne;
@@ -1242,139 +1279,432 @@ __global__ void __launch_bounds__(kCompactThreads) kb_compact_inject(const Dev* 
 // ---- the fused step: one block per replica, every phase inside the block ----------
 //
 // For replicas small enough that one block carries their whole step, the
-// phases above run back to back inside one kernel with __syncthreads between
-// them, for many steps per launch.  The phase bodies are the ones the
-// separate kernels call, over the same index ranges, with a block-uniform
-// loop (every thread runs the same iterations, so the warp-level sums in
-// move_body see full warps); __syncthreads orders their global-memory writes
-// as the kernel boundaries do.  Only the pair sum differs in form.
+// phases run back to back inside one kernel, for many steps per launch.  What
+// bounds it is the chain of round trips and barriers, so the carriers' state
+// lives in shared memory (win entries per species; a replica that outgrows it
+// goes on in its global arrays), a carrier's two potentials are summed and
+// decided by the same threads without a pass in between, and contested sites
+// are settled by comparing the accepted moves of the list instead of claiming
+// sites in memory.  1024 solar cells of 128x128 after 2000 steps of burn-in: 53 us
+// a step, with the phases as separate passes over global arrays 81.  At that load
+// the blocks issue 1.7 instructions a clock and an SM (MUFU 24%, FMA 21% busy):
+// carriers differ between replicas, and the SM with the most sets the time.
+// Holding 5-8 blocks an SM instead of 4 (fewer registers) changed nothing.
+//
+// It takes the separate kernels' decisions: the same draws, the same rules, FP32
+// runs of kSUB sources of one charge class in list order folded into FP64
+// (r^2 - 1/2 exact, MUFU rsqrt, predicated FFMA), decisions within the guard
+// band of them redone in FP64.  Only the order of the FP64 additions differs.
 
+// A replica's arrays, in shared memory or global.
+struct StepArrays {
+    int32_t *es, *hs;   // sites
+    int32_t *ef, *hf;   // proposals; after the decisions -1 stays, -2 recombined,
+                        // else where the carrier goes
+    float4 *se, *sh;    // source records {-2x, -2y, -2z, |s|^2 - 1/2}
+    int32_t* flagged;   // decisions for the FP64 guard
+    int32_t *rch, *rcl; // recombination: an electron's hole; a hole's lowest electron
+};
+// Shared-memory bytes per carrier of a species' window, both species.
+constexpr int kStepBytes = 2 * (4 + 4 + 16) + 8 + 4 + 4;
 
-// The replica's pair sum inside the block: for every target the arithmetic of
-// pair_tile with a single source split -- runs of kSUB sources in FP32 (r^2 - 1/2
-// exact, MUFU rsqrt, predicated FFMA), each run folded into FP64 in source
-// order, |run sum| added to the FP32 norm -- so the partials equal those of the
-// pair kernel with one split bit for bit.  One target per thread at a time:
-// every thread reads the same source record at a time (one broadcast load per
-// warp, an L1 hit after the first warp).  Carrying 2-4 targets per thread
-// through the source loop measured slower here (fewer threads busy, more
-// registers).  A charge class is padded to whole chunks with records of
-// charge 0; its runs past the class's live charges add exact zeros and are
-// skipped.
-__device__ void fused_pair_body(const Dev& D) {
-    const int ne = D.cnt[I_NE], nh = D.cnt[I_NH];
-    const int nd = D.dq != 0 ? D.nd : 0;
-    const int pe = (ne + CH - 1) / CH * CH, ph = (nh + CH - 1) / CH * CH;
-    const int start[3] = {0, pe, pe + ph}, count[3] = {ne, nh, nd};
-    const int t = 2 * (ne + nh);
-    const int tpad = D.cnt[I_TPAD];
-    const float4* geo = D.geo;
-    const float2* qq = D.qq;
-    const float* gtab = D.gtab;
-    const int gtab_k = D.gtab_k, gauss = D.gauss;
-    const unsigned ulim = __float_as_uint((float)D.cutoff2 - 0.5f);
-    for (int g = threadIdx.x; g < D.nterms * t; g += blockDim.x) {
-        const int slot = g / t;
-        const int p = slot * tpad + (g - slot * t);
-        const float4 tg = D.tgt[p];
-        double acc64 = 0.0;
-        float nrm = 0.f;
-        for (int c = 0; c < 3; ++c) {
-            const int s1 = start[c] + count[c];
-            for (int r0 = start[c]; r0 < s1; r0 += kSUB) {
-                const int r1 = min(r0 + kSUB, s1);
-                float acc = 0.f;
-                for (int j = r0; j < r1; ++j) {
-                    const float4 g0 = geo[2 * j], g1 = geo[2 * j + 1];
-                    float u = __fadd_rn(g1.z, tg.w);  // d + |t|^2
-                    u = __fmaf_rn(tg.x, g0.x, u);
-                    u = __fmaf_rn(tg.y, g0.z, u);
-                    u = __fmaf_rn(tg.z, g1.x, u);     // r^2 - 1/2, exact
-                    const float r2 = __fadd_rn(u, 0.5f);
-                    float w = rsqrt_mufu(r2);
-                    if (gauss) {
-                        const int ix = min(__float_as_int(r2 + 8388608.f) & 0x7fffff, gtab_k);
-                        w = fminf(gtab[ix], w);
-                    }
-                    fma_if_below(acc, qq[j].x, w, __float_as_uint(u), ulim);
-                }
-                acc64 += (double)acc;
-                nrm += fabsf(acc);
-            }
+// Grid::neighborsSite at range 1 in its order (neighbors()), as a rank: the
+// nb-th neighbour (drains last) for nb below the count, which is returned.
+__device__ __forceinline__ int neighbors1(const Dev& D, int site, int x, int y, int z,
+                                          bool electron, int nb, int* out) {
+    int n = 0, f = -1;
+    auto take = [&](bool on, int s) {
+        if (on) {
+            if (n == nb) f = s;
+            ++n;
         }
-        D.part[p] = acc64;
-        D.part_norm[p] = nrm;
+    };
+    take(x > 0, site - 1);
+    take(x < D.X - 1, site + 1);
+    take(y > 0, site - D.X);
+    take(y < D.Y - 1, site + D.X);
+    take(z > 0, site - D.XY);
+    take(z < D.Z - 1, site + D.XY);
+    take(x == 0, D.V + (electron ? E_DRAIN_L : H_DRAIN_L));
+    take(x == D.X - 1, D.V + (electron ? E_DRAIN_R : H_DRAIN_R));
+    *out = f;
+    return n;
+}
+
+__device__ __forceinline__ float4 step_record(const Dev& D, int site) {
+    int x, y, z;
+    xyz(D, site, x, y, z);
+    return make_float4(-2.f * x, -2.f * y, -2.f * z, (float)(x * x + y * y + z * z) - 0.5f);
+}
+
+// The sums of one carrier's two targets over runs part, part + split, ... of the
+// n sources of one charge class.
+__device__ __forceinline__ void step_class_sum(const float4* src, int n, float q, int part, int split,
+                                               const float4 ta, const float4 tb, unsigned ulim,
+                                               const float* gtab, int gtab_k, int gauss,
+                                               double (&v)[2], float (&m)[2]) {
+    for (int r0 = part * kSUB; r0 < n; r0 += split * kSUB) {
+        const int r1 = min(r0 + kSUB, n);
+        float acc[2] = {0.f, 0.f};
+#pragma unroll 4
+        for (int j = r0; j < r1; ++j) {
+            const float4 g = src[j];
+            const float ua = __fmaf_rn(ta.z, g.z, __fmaf_rn(ta.y, g.y,
+                                       __fmaf_rn(ta.x, g.x, __fadd_rn(g.w, ta.w))));
+            const float ub = __fmaf_rn(tb.z, g.z, __fmaf_rn(tb.y, g.y,
+                                       __fmaf_rn(tb.x, g.x, __fadd_rn(g.w, tb.w))));
+            const float ra = __fadd_rn(ua, 0.5f), rb = __fadd_rn(ub, 0.5f);
+            float wa = rsqrt_mufu(ra), wb = rsqrt_mufu(rb);
+            if (gauss) {
+                wa = fminf(gtab[min(__float_as_int(ra + 8388608.f) & 0x7fffff, gtab_k)], wa);
+                wb = fminf(gtab[min(__float_as_int(rb + 8388608.f) & 0x7fffff, gtab_k)], wb);
+            }
+            fma_if_below(acc[0], q, wa, __float_as_uint(ua), ulim);
+            fma_if_below(acc[1], q, wb, __float_as_uint(ub), ulim);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            v[k] += (double)acc[k];
+            m[k] += fabsf(acc[k]);
+        }
     }
 }
 
-#define LGM_BLOCK_LOOP(BOUND, CALL)                                                     \
-    for (int base_ = 0; base_ < (BOUND); base_ += (int)blockDim.x) {                  \
-        const int i = base_ + (int)threadIdx.x;                                       \
-        CALL;                                                                         \
-    }
-
-// Block b advances replica list[b] by `steps` steps.  `recomb` is the batch's
-// flag (the recombination phases run for every replica of a batch in which any
-// replica recombines, as the separate kernels do).  The replica's descriptor
-// is copied to shared memory once; each phase loops over the live charges
-// counted at the phase's start, not over the capacity.
+// Block b advances replica list[b] by `steps` steps.  recomb: the batch's flag.
 template <int NT>
-__global__ void __launch_bounds__(NT) kb_fused(const Dev* R, const int* list, int steps, int recomb) {
-    __shared__ double2 red[NT];
+__global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) kb_fused(const Dev* R, const int* list, int steps, int recomb,
+                                               int win) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ double2 red[32];
     __shared__ int warp_sums[32];
     __shared__ Dev sD;
+    __shared__ StepArrays sA;
+    __shared__ int32_t s_cnt[I_NUM];
+    __shared__ unsigned long long s_ctr[C_NUM];
+    const Dev& G = R[list[blockIdx.x]];
+    const int tid = threadIdx.x;
     {
         static_assert(sizeof(Dev) % 4 == 0, "word copy");
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&R[list[blockIdx.x]]);
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(&G);
         uint32_t* dst = reinterpret_cast<uint32_t*>(&sD);
-        for (int w = threadIdx.x; w < (int)(sizeof(Dev) / 4); w += NT) dst[w] = src[w];
+        for (int w = tid; w < (int)(sizeof(Dev) / 4); w += NT) dst[w] = src[w];
+        for (int i = tid; i < I_NUM; i += NT) s_cnt[i] = G.cnt[i];
+        for (int i = tid; i < C_NUM; i += NT) s_ctr[i] = G.ctr[i];
+    }
+    __syncthreads();
+    bool local = s_cnt[I_NE] + 2 <= win && s_cnt[I_NH] + 2 <= win && !sD.balance;
+    if (tid == 0) {
+        sD.cnt = s_cnt;
+        sD.ctr = s_ctr;
+        float4* f = reinterpret_cast<float4*>(smem);
+        int32_t* p = reinterpret_cast<int32_t*>(f + 2 * win);
+        if (local) {
+            sA = StepArrays{p, p + win, p + 2 * win, p + 3 * win, f, f + win, p + 4 * win,
+                            p + 6 * win, p + 7 * win};
+            sD.e_site = sA.es;
+            sD.h_site = sA.hs;
+        } else {
+            sA = StepArrays{G.e_site, G.h_site, G.e_f, G.h_f, G.geo, G.geo + G.cap_e, G.flagged,
+                            G.e_rch, G.rclaim};
+        }
     }
     __syncthreads();
     const Dev& D = sD;
     const int nd = D.dq != 0 ? D.nd : 0;
+    if (local) {
+        for (int i = tid; i < s_cnt[I_NE]; i += NT) sA.es[i] = G.e_site[i];
+        for (int i = tid; i < s_cnt[I_NH]; i += NT) sA.hs[i] = G.h_site[i];
+        for (int i = tid; i < win; i += NT) sA.rcl[i] = INT_MAX;
+    }
+    // charged defects stay where they are: their records once, behind the carriers'
+    float4* sd = G.geo + G.cap_e + G.cap_h;
+    if (D.coulomb)
+        for (int i = tid; i < nd; i += NT) sd[i] = step_record(D, D.defects[i]);
+    __syncthreads();
+
     for (int s = 0; s < steps; ++s) {
-        int ne = D.cnt[I_NE], nh = D.cnt[I_NH];
-        LGM_BLOCK_LOOP(max(1, ne + nh), choose_body(D, i))
-        __syncthreads();
-        if (D.coulomb) {
-            const int nsrc = (ne + CH - 1) / CH * CH + (nh + CH - 1) / CH * CH +
-                             (nd + CH - 1) / CH * CH;
-            const int tpad = (2 * (ne + nh) + 63) / 64 * 64;
-            LGM_BLOCK_LOOP(max(nsrc, tpad), pack_body(D, i))
+        const int ne = s_cnt[I_NE], nh = s_cnt[I_NH], n = ne + nh;
+        const uint32_t step = (uint32_t)s_cnt[I_STEP];
+        if (local && (ne + 2 > win || nh + 2 > win)) {
+            // outgrown: on in the global arrays
+            for (int i = tid; i < ne; i += NT) G.e_site[i] = sA.es[i];
+            for (int i = tid; i < nh; i += NT) G.h_site[i] = sA.hs[i];
             __syncthreads();
-            fused_pair_body(D);
-            __syncthreads();
-            LGM_BLOCK_LOOP(2 * (ne + nh), finalize_body(D, i))
-            __syncthreads();
-        }
-        LGM_BLOCK_LOOP(ne + nh, decide_body(D, i))
-        __syncthreads();
-        if (D.coulomb) {
-            guard_body(D, 0, 1, red);
+            if (tid == 0) {
+                sA = StepArrays{G.e_site, G.h_site, G.e_f, G.h_f, G.geo, G.geo + G.cap_e, G.flagged,
+                                G.e_rch, G.rclaim};
+                sD.e_site = G.e_site;
+                sD.h_site = G.h_site;
+            }
+            local = false;
             __syncthreads();
         }
+        const StepArrays A = sA;
+        // ---- proposals (choose_body) and source records
+        for (int i = tid; i < n; i += NT) {
+            const bool e = i < ne;
+            const int k = e ? i : i - ne;
+            const int site = (e ? A.es : A.hs)[k];
+            const Philox4 r = draw(D, step, (uint32_t)k, e ? RNG_CHOOSE_E : RNG_CHOOSE_H);
+            int f, x, y, z;
+            xyz(D, site, x, y, z);
+            if (D.hr == 1) {
+                const int m = neighbors1(D, site, x, y, z, e, -1, &f);
+                neighbors1(D, site, x, y, z, e, (int)uint_below(r.w[0], (uint32_t)m), &f);
+            } else {
+                int nb[40];
+                const int m = neighbors(D, site, e, nb, D.hr);
+                f = nb[uint_below(r.w[0], (uint32_t)m)];
+            }
+            (e ? A.ef : A.hf)[k] = f;
+            if (D.coulomb)
+                (e ? A.se : A.sh)[k] =
+                    make_float4(-2.f * x, -2.f * y, -2.f * z, (float)(x * x + y * y + z * z) - 0.5f);
+        }
+        if (tid == 0) {
+            s_cnt[I_NE0] = ne;
+            s_cnt[I_NH0] = nh;
+            s_cnt[I_NFLAG] = 0;
+            s_cnt[I_REMOVED] = 0;
+            s_cnt[I_FIRST_E] = INT_MAX;
+            s_cnt[I_FIRST_H] = INT_MAX;
+            s_ctr[C_PROPOSALS] += (unsigned)n;
+        }
+        __syncthreads();
+        // ---- potentials and decisions (decide_body): `split` threads per carrier
+        int split = 1;
+        while (D.coulomb && split < 8 && 2 * split * n <= NT) split *= 2;
+        const int part = tid & (split - 1);
+        for (int c0 = 0; c0 < n; c0 += NT / split) {
+            const int i = c0 + tid / split;
+            const bool on = i < n, e = i < ne;
+            const int k = e ? i : i - ne;
+            int site = 0, f = 0;
+            uint8_t type = T_DEFECT;
+            if (on) {
+                site = (e ? A.es : A.hs)[k];
+                f = (e ? A.ef : A.hf)[k];
+                type = (e ? D.et : D.ht)[f];
+                if (D.confine && f < D.V && type == T_EMPTY && D.phase[f] != (e ? 1 : 0)) type = T_DEFECT;
+            }
+            const double q = e ? -1.0 : 1.0;
+            double dpot = 0.0, b1 = 0.0, b2 = 0.0;
+            if (on && type == T_EMPTY && part == 0) {
+                dpot = D.pot[f] - D.pot[site];
+                if (D.coulomb) {
+                    b1 = binding(D, e, site);
+                    b2 = binding(D, e, f);
+                }
+            }
+            double V[2] = {0.0, 0.0}, M[2] = {0.0, 0.0};
+            if (D.coulomb) {  // (a target that is not empty needs no potential)
+                if (on && type == T_EMPTY) {
+                    const unsigned ulim = __float_as_uint((float)D.cutoff2 - 0.5f);
+                    int xa, ya, za, xb, yb, zb;
+                    xyz(D, site, xa, ya, za);
+                    xyz(D, f, xb, yb, zb);
+                    for (int term = 0; term < 3; ++term) {
+                        if (!(D.terms & (1u << term))) continue;
+                        const int pa = term == 0 ? xa : term == 1 ? -1 - xa : 2 * D.X - 1 - xa;
+                        const int pb = term == 0 ? xb : term == 1 ? -1 - xb : 2 * D.X - 1 - xb;
+                        const float4 ta = make_float4((float)pa, (float)ya, (float)za,
+                                                      (float)(pa * pa + ya * ya + za * za));
+                        const float4 tb = make_float4((float)pb, (float)yb, (float)zb,
+                                                      (float)(pb * pb + yb * yb + zb * zb));
+                        double v[2] = {0.0, 0.0};
+                        float m[2] = {0.f, 0.f};
+                        step_class_sum(A.se, ne, -1.f, part, split, ta, tb, ulim, D.gtab, D.gtab_k,
+                                       D.gauss, v, m);
+                        step_class_sum(A.sh, nh, 1.f, part, split, ta, tb, ulim, D.gtab, D.gtab_k,
+                                       D.gauss, v, m);
+                        if (nd)
+                            step_class_sum(sd, nd, (float)D.dq, part, split, ta, tb, ulim, D.gtab,
+                                           D.gtab_k, D.gauss, v, m);
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            V[t] = term == 0 ? v[t] : V[t] - v[t];
+                            M[t] += (double)m[t];
+                        }
+                    }
+                }
+                for (int o = 1; o < split; o <<= 1)
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        V[t] += __shfl_xor_sync(0xffffffffu, V[t], o);
+                        M[t] += __shfl_xor_sync(0xffffffffu, M[t], o);
+                    }
+            }
+            if (!on || part != 0) continue;  // (the loop's trip count is the block's)
+            int32_t out = O_OCCUPIED;
+            bool acc = false, flag = false;
+            double de = 0.0;
+            if (type == T_EMPTY) {
+                const double c = coupling_of(D, site, f);
+                const Philox4 r = draw(D, step, (uint32_t)k, e ? RNG_DECIDE_E : RNG_DECIDE_H);
+                const double u = unit_double(r.w[0], r.w[1]);
+                double pd = dpot * q;
+                if (D.coulomb) {
+                    const double p1 = D.prefactor * V[0] + b1;
+                    const double p2 = D.prefactor * V[1] - D.sI100 * q + b2;
+                    de = q * (p2 - p1);
+                    pd += de;
+                    if (u < c) {
+                        const double tau = log(c / u) / D.beta;
+                        const double g = D.guard * (D.prefactor * M[0] + D.prefactor * M[1]) +
+                                         1e-12 * (1.0 + fabs(pd));
+                        if (fabs(pd - tau) <= g) flag = true;
+                        else acc = pd < tau;
+                    }
+                } else {
+                    acc = metropolis(pd, D.beta, c, u);
+                }
+                if (flag) A.flagged[atomicAdd(&s_cnt[I_NFLAG], 1)] = i;
+                out = flag ? -1 : acc ? O_MET_ACCEPT : O_MET_REJECT;
+            } else if (type == T_DRAIN) {
+                const int which = f - D.V;
+                const int agent = e ? (which == E_DRAIN_L ? 0 : 1) : (which == H_DRAIN_L ? 2 : 3);
+                atomicAdd(&s_ctr[2 * (4 + agent)], 1ull);
+                const Philox4 r = draw(D, step, (uint32_t)k, e ? RNG_DECIDE_E : RNG_DECIDE_H);
+                acc = D.rate_drain[agent] > unit_double(r.w[0], r.w[1]);
+                if (acc) atomicAdd(&s_ctr[2 * (4 + agent) + 1], 1ull);
+                out = acc ? O_DRAIN_ACCEPT : O_DRAIN_REJECT;
+            }
+            if (!acc && !flag) (e ? A.ef : A.hf)[k] = -1;
+            if (s == steps - 1) {
+                G.outcome[i] = out;
+                G.de[i] = de;
+            }
+        }
+        __syncthreads();
+        // ---- the guard: queued decisions in FP64, the whole block on each
+        const int nflag = s_cnt[I_NFLAG];
+        for (int w = 0; w < nflag; ++w) {
+            const int i = A.flagged[w];
+            const bool e = i < ne;
+            const int k = e ? i : i - ne;
+            const int site = (e ? A.es : A.hs)[k], f = (e ? A.ef : A.hf)[k];
+            const double2 t = fp64_potential2(D, ne, nh, site, f, 0, n + nd, red);
+            if (tid == 0) {
+                const double q = e ? -1.0 : 1.0;
+                const double p1 = D.prefactor * t.x + binding(D, e, site);
+                const double p2 = D.prefactor * t.y - D.sI100 * q + binding(D, e, f);
+                const double de = q * (p2 - p1);
+                const Philox4 r = draw(D, step, (uint32_t)k, e ? RNG_DECIDE_E : RNG_DECIDE_H);
+                const bool acc = metropolis((D.pot[f] - D.pot[site]) * q + de, D.beta,
+                                            coupling_of(D, site, f), unit_double(r.w[0], r.w[1]));
+                if (!acc) (e ? A.ef : A.hf)[k] = -1;
+                s_ctr[C_GUARD] += 1;
+                if (s == steps - 1) {
+                    G.outcome[i] = acc ? O_MET_ACCEPT : O_MET_REJECT;
+                    G.de[i] = de;
+                }
+            }
+        }
+        if (nflag > 0) __syncthreads();
+        // ---- recombination (recomb_*_body); a hole's index by looking its site up
         if (recomb) {
-            LGM_BLOCK_LOOP(nh, hmap_body(D, i, true))
+            for (int i = tid; i < ne; i += NT) {
+                const int site = A.es[i];
+                int at = -1, cnt = 0;
+                const Philox4 r = draw(D, step, (uint32_t)i, RNG_RECOMB);
+                if (D.rec_range <= 1) {
+                    int cand[7];
+                    uint8_t type[7];
+                    int m = 1;
+                    cand[0] = site;
+                    if (D.rec_range == 1) {
+                        int x, y, z;
+                        xyz(D, site, x, y, z);
+                        m = 7;
+                        cand[1] = x > 0 ? site - 1 : -1;
+                        cand[2] = x < D.X - 1 ? site + 1 : -1;
+                        cand[3] = y > 0 ? site - D.X : -1;
+                        cand[4] = y < D.Y - 1 ? site + D.X : -1;
+                        cand[5] = z > 0 ? site - D.XY : -1;
+                        cand[6] = z < D.Z - 1 ? site + D.XY : -1;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 7; ++j) type[j] = j < m && cand[j] >= 0 ? D.ht[cand[j]] : T_EMPTY;
+#pragma unroll
+                    for (int j = 0; j < 7; ++j) cnt += type[j] == T_HOLE;
+                    if (cnt > 0) {
+                        int pick = (int)uint_below(r.w[0], (uint32_t)cnt);
+#pragma unroll
+                        for (int j = 0; j < 7; ++j)
+                            if (type[j] == T_HOLE && pick-- == 0) at = cand[j];
+                    }
+                } else {
+                    int nb[40], cand[48];
+                    if (D.ht[site] == T_HOLE) cand[cnt++] = site;
+                    const int m = neighbors(D, site, true, nb, D.rec_range);
+                    for (int j = 0; j < m; ++j)
+                        if (D.ht[nb[j]] == T_HOLE) cand[cnt++] = nb[j];
+                    if (cnt > 0) at = cand[uint_below(r.w[0], (uint32_t)cnt)];
+                }
+                int hk = -1;
+                if (at >= 0)
+                    for (int j = 0; j < nh; ++j)
+                        if (A.hs[j] == at) hk = j;
+                A.rch[i] = hk;
+                if (hk >= 0 && D.rec_rate > unit_double(r.w[1], r.w[2])) atomicMin(&A.rcl[hk], i);
+            }
             __syncthreads();
-            LGM_BLOCK_LOOP(ne, recomb_propose_body(D, i))
+            for (int i = tid; i < ne; i += NT) {
+                const int hk = A.rch[i];
+                if (hk < 0) continue;
+                const int w = A.rcl[hk];
+                if (w == INT_MAX || i <= w) atomicAdd(&s_ctr[C_RECOMB], 1ull);
+                if (i == w) {
+                    atomicAdd(&s_ctr[C_RECOMB + 1], 1ull);
+                    A.ef[i] = -2;
+                    A.hf[hk] = -2;
+                }
+            }
             __syncthreads();
-            LGM_BLOCK_LOOP(ne, recomb_resolve_body(D, i))
-            __syncthreads();
-            LGM_BLOCK_LOOP(max(ne, nh), recomb_reset_body(D, i))
-            __syncthreads();
+            for (int i = tid; i < ne; i += NT)
+                if (A.rch[i] >= 0) A.rcl[A.rch[i]] = INT_MAX;
         }
-        LGM_BLOCK_LOOP(ne + nh, claim_body(D, i))
-        __syncthreads();
-        LGM_BLOCK_LOOP(ne + nh, move_body(D, i))
-        __syncthreads();
-        LGM_BLOCK_LOOP(ne + nh, unclaim_body(D, i))
+        // ---- completeTick in list order (claim_body, move_body): the lowest
+        // index among a species' accepted moves to a site takes it
+        for (int i = tid; i < n; i += NT) {
+            const bool e = i < ne;
+            const int k = e ? i : i - ne;
+            const int32_t* to = e ? A.ef : A.hf;
+            const int f = to[k];
+            if (f == -1) continue;
+            int32_t* sites = e ? A.es : A.hs;
+            uint8_t* own = e ? D.et : D.ht;
+            const int site = sites[k];
+            if (f == -2 || f >= D.V) {  // recombined, or into a drain
+                own[site] = T_EMPTY;
+                sites[k] = -1;
+                s_cnt[I_REMOVED] = 1;
+                atomicMin(&s_cnt[e ? I_FIRST_E : I_FIRST_H], k);
+                if (f >= 0) atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
+                continue;
+            }
+            bool mine = true;
+#pragma unroll 8
+            for (int j = 0; j < k; ++j) mine &= to[j] != f;
+            if (mine) {
+                own[site] = T_EMPTY;
+                own[f] = e ? T_ELECTRON : T_HOLE;
+                sites[k] = f;
+                atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
+            }
+        }
         __syncthreads();
         compact_inject_body(D, warp_sums, reinterpret_cast<double*>(red));
         __syncthreads();
     }
+    // ---- back to the replica's own arrays
+    if (local) {
+        for (int i = tid; i < s_cnt[I_NE]; i += NT) G.e_site[i] = sA.es[i];
+        for (int i = tid; i < s_cnt[I_NH]; i += NT) G.h_site[i] = sA.hs[i];
+    }
+    for (int i = tid; i < I_NUM; i += NT) G.cnt[i] = s_cnt[i];
+    for (int i = tid; i < C_NUM; i += NT) G.ctr[i] = s_ctr[i];
 }
-// Block sizes of the fused step: small replicas fill 128 threads, larger 256.
-constexpr int kFusedSmallCharges = 512;
 
 // ---- host side -------------------------------------------------------------------
 
@@ -2316,6 +2646,9 @@ constexpr int kFusedMaxCharges = 2048;
 // Steps per launch of the fused kernel when no replica needs the per-phase
 // kernels (bounds the length of one launch).
 constexpr int kFusedStepsPerLaunch = 1000;
+// The fused step's window, and the shared memory of an SM that its blocks share.
+constexpr int kStepWindow = 1024;
+constexpr int kStepSmem = 200 * 1024;
 
 }  // namespace
 
@@ -2339,7 +2672,8 @@ struct lgm_kmc_batch {
     // replicas on the fused step and on the per-phase kernels
     int fused_max = kFusedMaxCharges;
     bool started = false;  // a step has run: the partition is fixed
-    bool fused_small = false;  // every fused replica fits the 128-thread block
+    int fused_threads = 256;   // the fused step's block size
+    int fused_win = 0;         // carriers per species it keeps in shared memory
     bool fused_set = false;    // the caller set the bound: capacity alone decides
     std::vector<int> fused, classic;
     int *d_fused = nullptr, *d_classic = nullptr;
@@ -2458,12 +2792,15 @@ lgm_status enqueue_batch_pair(lgm_kmc_batch* b, cudaStream_t st) {
     return enqueue_batch_items(b, st);
 }
 
+using FusedFn = void (*)(const Dev*, const int*, int, int, int);
+FusedFn fused_fn(int threads) {
+    return threads <= 128 ? kb_fused<128> : kb_fused<256>;
+}
+
 void launch_fused(const lgm_kmc_batch* b, cudaStream_t st, int steps) {
     const int n = (int)b->fused.size();
-    if (b->fused_small)
-        kb_fused<128><<<n, 128, 0, st>>>(b->d_reps, b->d_fused, steps, b->recomb);
-    else
-        kb_fused<256><<<n, 256, 0, st>>>(b->d_reps, b->d_fused, steps, b->recomb);
+    fused_fn(b->fused_threads)<<<n, b->fused_threads, (size_t)b->fused_win * kStepBytes, st>>>(
+        b->d_reps, b->d_fused, steps, b->recomb, b->fused_win);
 }
 
 // The fused replicas' step on the aux stream, forked from and joined back to
@@ -2590,9 +2927,21 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
         const bool fits = D.cap_e + D.cap_h <= b->fused_max && (b->fused_set || all_fit);
         (fits ? b->fused : b->classic).push_back(r);
     }
-    b->fused_small = true;
-    for (int r : b->fused)
-        b->fused_small &= b->hD[r].cap_e + b->hD[r].cap_h <= kFusedSmallCharges;
+    if (!b->fused.empty()) {
+        const int per_sm = ((int)b->fused.size() + b->reps[0]->sm_count - 1) / b->reps[0]->sm_count;
+        int cap = 1;
+        for (int r : b->fused) cap = std::max({cap, b->hD[r].cap_e, b->hD[r].cap_h});
+        b->fused_win = std::max(128, std::min({cap + 2, kStepWindow,
+                                               kStepSmem / per_sm / kStepBytes}));
+        // Up to two blocks an SM 256 threads are the faster ones (200 replicas of
+        // 128x128: 18 us a step against 22), beyond that 128 (1024: 62 against 72).
+        b->fused_threads = per_sm <= 2 ? 256 : 128;
+        // the limit is the function's, not the batch's: always the largest window
+        const cudaError_t e = cudaFuncSetAttribute(fused_fn(b->fused_threads),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   kStepWindow * kStepBytes);
+        if (e != cudaSuccess) return bfail(b, LGM_ERR_CUDA, "shared memory of the fused step");
+    }
     for (int r : b->fused) b->hD[r].sorted = 0;  // the fused step keeps the list order
     for (int r : b->classic) b->hD[r].sorted = b->hD[r].coulomb;
     // culled pair sums for the per-phase replicas with room for enough chunks

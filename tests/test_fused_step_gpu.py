@@ -1,0 +1,89 @@
+"""The fused kMC step at the edges of its shared-memory window, against single
+replicas (the per-phase kernels), and the electrode sources' order against the
+oracle on lattices one and two sites wide."""
+import numpy as np
+import pytest
+
+import langmuir_b200 as L
+from oracle.kmc_setup import independent_world, oracle_for
+
+WINDOW = 1024  # carriers per species held in shared memory, at most
+
+
+def params(**keys):
+    base = dict(simulation_type="transistor", random_seed=11, seed_charges=1.0, coulomb_carriers=1,
+                iterations_real=1000, iterations_print=10, grid_x=64, grid_y=64, grid_z=2,
+                electron_percentage=0.15, hole_percentage=0.02, electrostatic_cutoff=10,
+                voltage_right=1.0, e_source_l_rate=1.0, e_source_r_rate=1.0, e_drain_l_rate=0.01,
+                e_drain_r_rate=0.01, h_drain_l_rate=0.5)
+    base.update(keys)
+    p = L.Params.default()
+    for k, v in base.items():
+        p.set(k, v)
+    return p
+
+
+def inner_sites(n, seed):
+    """n distinct sites off the electrodes' faces of a 64x64x2 lattice."""
+    s = np.arange(64 * 64 * 2)
+    s = s[(s % 64 > 0) & (s % 64 < 63)]
+    return np.random.default_rng(seed).choice(s, n, replace=False).astype(np.int32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("start", [WINDOW - 10, WINDOW - 2, WINDOW + 40])
+def test_window_edges_match_single_replicas(start):
+    p, steps = params(), 30
+    e, h = inner_sites(start, 3), inner_sites(40, 4)
+    with L.KMCBatch([p], replica0=9, fused_max_charges=4096) as b:
+        assert b.fused_count == 1
+        b.replica(0).set_carriers(e, h)
+        b.run(steps)
+        (e1, h1), s1 = b.replica(0).carriers(), b.replica(0).stats()
+    with L.KMC(p, replica=9) as k:
+        k.set_carriers(e, h)
+        k.run(steps)
+        (e2, h2), s2 = k.carriers(), k.stats()
+    assert len(e2) > WINDOW - 2  # past the window by the end
+    np.testing.assert_array_equal(e1, e2)
+    np.testing.assert_array_equal(h1, h2)
+    assert s1["counters"] == s2["counters"]
+
+
+@pytest.mark.gpu
+def test_a_small_batch_leaves_a_large_one_its_window():
+    big, small = params(), params(electron_percentage=0.005, hole_percentage=0.005)
+    e, h = inner_sites(900, 3), inner_sites(40, 4)
+    out = []
+    for between in (False, True):
+        with L.KMCBatch([big], replica0=2, fused_max_charges=4096) as b:
+            b.replica(0).set_carriers(e, h)
+            b.run(3)
+            if between:
+                with L.KMCBatch([small]) as c:
+                    c.run(3)
+            b.run(3)
+            out.append(b.replica(0).carriers())
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("x", [1, 2])
+def test_sources_on_narrow_lattices_match_oracle(oracle_mod, x):
+    """Both electrodes' faces are one face when the lattice is one site wide."""
+    p = params(grid_x=x, grid_y=5, grid_z=2, electron_percentage=0.8, hole_percentage=0.8,
+               seed_charges=0.0, h_source_l_rate=1.0, h_source_r_rate=1.0)
+    with L.KMC(p, replica=4) as k:
+        st = k.stats()
+        e0, h0 = k.carriers()
+        orc = oracle_for(oracle_mod, p, independent_world(p, 4), e0, h0, st["max_electrons"],
+                         st["max_holes"], replica=4)
+        for _ in range(40):
+            orc.step()
+        k.run(40)
+        e, h = k.carriers()
+        e_o, h_o = orc.carriers()
+        np.testing.assert_array_equal(e, e_o)
+        np.testing.assert_array_equal(h, h_o)
+        np.testing.assert_array_equal(np.array(k.stats()["counters"], np.uint64), orc.counters)
