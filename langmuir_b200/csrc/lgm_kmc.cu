@@ -1370,10 +1370,9 @@ __device__ __forceinline__ void step_class_sum(const float4* src, int n, float q
     }
 }
 
-// Block b advances replica list[b] by `steps` steps.  recomb: the batch's flag.
+// The block advances replica G by `steps` steps.
 template <int NT>
-__global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) kb_fused(const Dev* R, const int* list, int steps, int recomb,
-                                               int win) {
+__device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb, int win) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double2 red[32];
     __shared__ int warp_sums[32];
@@ -1381,7 +1380,6 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) kb_fused(const Dev* R, 
     __shared__ StepArrays sA;
     __shared__ int32_t s_cnt[I_NUM];
     __shared__ unsigned long long s_ctr[C_NUM];
-    const Dev& G = R[list[blockIdx.x]];
     const int tid = threadIdx.x;
     {
         static_assert(sizeof(Dev) % 4 == 0, "word copy");
@@ -1704,6 +1702,19 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2) kb_fused(const Dev* R, 
     }
     for (int i = tid; i < I_NUM; i += NT) G.cnt[i] = s_cnt[i];
     for (int i = tid; i < C_NUM; i += NT) G.ctr[i] = s_ctr[i];
+}
+
+// Block b advances replica list[b].  recomb: the batch's flag.
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2)
+kb_fused(const Dev* R, const int* list, int steps, int recomb, int win) {
+    fused_steps<NT>(R[list[blockIdx.x]], steps, recomb, win);
+}
+// A small standalone replica, one block.
+constexpr int kFusedAloneThreads = 512;
+__global__ void __launch_bounds__(kFusedAloneThreads)
+k_fused(const __grid_constant__ Dev D, int steps, int recomb, int win) {
+    fused_steps<kFusedAloneThreads>(D, steps, recomb, win);
 }
 
 // ---- host side -------------------------------------------------------------------
@@ -2089,6 +2100,32 @@ cudaError_t kl(void (*f)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t
     cfg.attrs = at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, f, static_cast<P>(args)...);
+}
+
+// Steps per launch of the fused kernel (bounds the length of one launch).
+constexpr int kFusedStepsPerLaunch = 1000;
+
+// A standalone replica takes the fused step when one block's sums take less
+// time than the separate kernels' launches, some 40 us a step whatever the
+// size.  With 512 threads a step takes about 6 us and 0.12 us per 1000 carriers x
+// sources x terms (us a step, fused and separate: 20 holes 5.6 and 37, 163 holes
+// 10.7 and 38, 490 carriers 33 and 40; 326 with both images, 319k, 47 and 40);
+// the Gaussian table makes a pair about 1.5 times as dear (458 carriers, 48 and
+// 46).  The room decides, not the carriers alive, so a replica keeps one form.
+// Culled replicas sum their sources in cell order and stay as they are.
+// 256 and 1024 threads took 11.5 and 16.2 us at 163 holes, 42 and 41 at 490.
+constexpr int kFusedAloneCharges = 512;
+constexpr double kFusedAlonePairs = 1 << 18;
+bool fused_alone(const lgm_kmc* k) {
+    const Dev& D = k->D;
+    const double n = D.cap_e + D.cap_h, sources = n + (D.dq != 0 ? D.nd : 0);
+    const double pairs = D.coulomb ? n * sources * D.nterms * (D.gauss ? 1.5 : 1.0) : 0.0;
+    return !k->pool && !D.culled && n <= kFusedAloneCharges && pairs <= kFusedAlonePairs;
+}
+void enqueue_fused_alone(const lgm_kmc* k, int steps) {
+    const int win = std::max(k->D.cap_e, k->D.cap_h) + 2;  // 33 KB at most
+    k_fused<<<1, kFusedAloneThreads, (size_t)win * kStepBytes, k->stream>>>(
+        k->D, steps, k->D.solar && k->D.rec_rate > 0, win);
 }
 
 // One step: kernels in order on k->stream (captured into the graph).
@@ -2485,7 +2522,12 @@ const char* lgm_kmc_last_error(const lgm_kmc* k) {
 lgm_status lgm_kmc_run(lgm_kmc* k, int32_t steps) {
     if (!k || steps < 0) return LGM_ERR_INVALID_ARGUMENT;
     KCUDA(k, cudaSetDevice(k->device));
-    if (!k->exec && steps > 0) {
+    const bool fused = fused_alone(k);
+    for (int done = 0; fused && done < steps; done += kFusedStepsPerLaunch) {
+        enqueue_fused_alone(k, std::min(kFusedStepsPerLaunch, steps - done));
+        KCUDA(k, cudaGetLastError());
+    }
+    if (!fused && !k->exec && steps > 0) {
         KCUDA(k, cudaStreamBeginCapture(k->stream, cudaStreamCaptureModeThreadLocal));
         lgm_status s = enqueue_step(k);
         cudaGraph_t g = nullptr;
@@ -2495,7 +2537,7 @@ lgm_status lgm_kmc_run(lgm_kmc* k, int32_t steps) {
         k->graph = g;
         KCUDA(k, cudaGraphInstantiate(&k->exec, g, 0));
     }
-    for (int i = 0; i < steps; ++i) KCUDA(k, cudaGraphLaunch(k->exec, k->stream));
+    for (int i = 0; !fused && i < steps; ++i) KCUDA(k, cudaGraphLaunch(k->exec, k->stream));
     KCUDA(k, cudaStreamSynchronize(k->stream));
     unsigned e = 0;
     KCUDA(k, cudaMemcpy(&e, k->D.err, sizeof e, cudaMemcpyDeviceToHost));
@@ -2643,9 +2685,6 @@ const int kChunksPerItem[] = {16, 48};
 // A batch whose replicas all have room for at most this many charges takes
 // the fused step by default (one block per replica).
 constexpr int kFusedMaxCharges = 2048;
-// Steps per launch of the fused kernel when no replica needs the per-phase
-// kernels (bounds the length of one launch).
-constexpr int kFusedStepsPerLaunch = 1000;
 // The fused step's window, and the shared memory of an SM that its blocks share.
 constexpr int kStepWindow = 1024;
 constexpr int kStepSmem = 200 * 1024;

@@ -87,3 +87,31 @@ def test_sources_on_narrow_lattices_match_oracle(oracle_mod, x):
         np.testing.assert_array_equal(e, e_o)
         np.testing.assert_array_equal(h, h_o)
         np.testing.assert_array_equal(np.array(k.stats()["counters"], np.uint64), orc.counters)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cap,keys", [
+    (1, dict()), (511, dict()), (512, dict()), (513, dict()),  # 512^2 pairs is the line
+    (295, dict(image_charges=3)), (296, dict(image_charges=3)),
+    (200, dict(defects_charge=1, defect_percentage=0.02))])
+def test_small_single_replicas_match_oracle(oracle_mod, cap, keys):
+    """Both sides of the line between the one-block step and the separate kernels."""
+    V = 64 * 64 * 2
+    p = params(hole_percentage=(cap + 0.5) / V, electron_percentage=0.0, e_source_l_rate=0.0,
+               e_source_r_rate=0.0, e_drain_l_rate=0.0, e_drain_r_rate=0.0, h_source_r_rate=0.7,
+               h_drain_l_rate=0.9, **keys)
+    with L.KMC(p, replica=6) as k:
+        st = k.stats()
+        assert st["max_holes"] == cap
+        e0, h0 = k.carriers()
+        orc = oracle_for(oracle_mod, p, independent_world(p, 6), e0, h0, st["max_electrons"],
+                         st["max_holes"], replica=6)
+        for n in (1, 7):  # a run after a run goes on where the first one ended
+            for _ in range(n):
+                orc.step()
+            k.run(n)
+            e, h = k.carriers()
+            e_o, h_o = orc.carriers()
+            np.testing.assert_array_equal(e, e_o)
+            np.testing.assert_array_equal(h, h_o)
+            np.testing.assert_array_equal(np.array(k.stats()["counters"], np.uint64), orc.counters)
