@@ -45,8 +45,10 @@ typedef int32_t lgm_status;
 typedef enum lgm_kind { LGM_POINT = 0, LGM_GAUSS = 1 } lgm_kind;
 
 /* Pair-sum arithmetic.  FP32C: FP32 terms, FP32 runs of up to 32 terms (16,
- * one source group, in the default variants) folded into FP64 accumulators.  FP64: every term in FP64 (the guard-band and
- * reference-precision path). */
+ * one source group, in the default variants) folded into FP64 accumulators.
+ * FP64: every term in FP64 (the guard-band and reference-precision path), from
+ * FP64 tables by r^2 up to cutoff 159, computed per pair beyond and in counting
+ * calls; lgm_launch_info reports variant -1. */
 typedef enum lgm_precision { LGM_PREC_FP32C = 0, LGM_PREC_FP64 = 1 } lgm_precision;
 
 /* How 1/r is formed in FP32C: MUFU reciprocal square root, or a per-r^2

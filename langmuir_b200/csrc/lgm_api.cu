@@ -394,6 +394,14 @@ __global__ void fill_zero(double* out, int t, const unsigned* err, unsigned* err
     if (g < t) out[g] = 0.0;
 }
 
+// The FP64 precision's tables are laid out up to this much shared memory of the
+// culled kernel (cutoff 159; its one CTA an SM is still the faster there).  128x128x8,
+// 2622 charges, host call with both images, tables and every term computed: cutoff
+// 50 65 us and 132, 90 85 and 134, 150 96 and 136; 400 charges at cutoff 158 62 and
+// 133.  The error against extended
+// precision halves (1.0e-15 to 5e-16 of the largest sum).
+constexpr size_t kF64TableSmem = 200 * 1024;
+
 // FP64 path: every term in double, 1/sqrt and erf of the CUDA runtime.
 // Sources staged in shared memory by plain loads; one thread per physical
 // target and split.
@@ -687,10 +695,9 @@ int splits_for(const lgm_ctx* c, int v, int fi, const Shape& sh, int* tiles_out)
 // Culled variant v: chunk boxes, the cull, the persistent pair kernel (one
 // wave of resident CTAs).  *splits_out = 0 tells the caller to finalize from
 // the item partials.
-lgm_status launch_culled(lgm_ctx* c, int kind, int v, const Shape& sh, const PairArgs& A,
+lgm_status launch_culled(lgm_ctx* c, int fi, int v, const Shape& sh, const PairArgs& A,
                          cudaStream_t st, int* splits_out) {
     const Variant& V = kVariants[v];
-    const int fi = fn_index(kind, c->cfg.path);
     const int TS = variant_tile(V);
     const int tiles = (sh.t_phys + TS - 1) / TS;
     const int grid = c->sm_count * std::max(1, c->bps[v][fi]);
@@ -773,10 +780,10 @@ lgm_status launch_culled(lgm_ctx* c, int kind, int v, const Shape& sh, const Pai
     return LGM_OK;
 }
 
-lgm_status launch_pair(lgm_ctx* c, int kind, int v, const Shape& sh, cudaStream_t st,
+lgm_status launch_pair(lgm_ctx* c, int kind, int path, int v, const Shape& sh, cudaStream_t st,
                        int* splits_out) {
     const lgm_config& cf = c->cfg;
-    const int fi = fn_index(kind, cf.path);
+    const int fi = fn_index(kind, path);
     if (kVariants[v].cull) {
         PairArgs A;
         A.geo = c->d_geo; A.qq = c->d_qq; A.n_chunks = sh.n_chunks; A.splits = 1;
@@ -785,17 +792,17 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int v, const Shape& sh, cudaStream_
         A.pad_group = sh.n_chunks * kGroupsPerChunk;
         A.c2 = (float)(cf.electrostatic_cutoff * cf.electrostatic_cutoff);
         A.err = c->d_err;
-        if (cf.path == LGM_PATH_TABLE64) {
+        if (path == LGM_PATH_TABLE64) {
             A.tab64 = kind == LGM_GAUSS ? c->d_gtab64 : c->d_rtab64;
             A.tab_k = c->rtab_k;  // both hold every r^2 <= c^2 (entries 0 and c^2 are 0)
-        } else if (cf.path == LGM_PATH_TABLE) {
+        } else if (path == LGM_PATH_TABLE) {
             A.tab = kind == LGM_GAUSS ? c->d_gtab : c->d_rtab;
             A.tab_k = kind == LGM_GAUSS ? c->gtab_k : c->rtab_k;
         } else {
             A.tab = c->d_gtab;
             A.tab_k = kind == LGM_GAUSS ? c->gtab_k : 0;
         }
-        return launch_culled(c, kind, v, sh, A, st, splits_out);
+        return launch_culled(c, fi, v, sh, A, st, splits_out);
     }
     int tiles;
     const int splits = splits_for(c, v, fi, sh, &tiles);
@@ -807,7 +814,7 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int v, const Shape& sh, cudaStream_
     A.tgt = c->d_tgt; A.t_phys = sh.t_phys; A.part = c->d_part;
     A.c2 = (float)(cf.electrostatic_cutoff * cf.electrostatic_cutoff);
     A.err = c->d_err;
-    if (cf.path == LGM_PATH_TABLE) {
+    if (path == LGM_PATH_TABLE) {
         A.tab = kind == LGM_GAUSS ? c->d_gtab : c->d_rtab;  // both hold every r^2 < c^2
         A.tab_k = kind == LGM_GAUSS ? c->gtab_k : c->rtab_k;
     } else {
@@ -838,10 +845,21 @@ int choose_variant(const lgm_ctx* c, int kind, const Shape& sh) {
     return v;
 }
 
+// The FP64 precision's sums: with their terms from the FP64 tables (d_rtab64,
+// laid out when the culled kernel's shared memory holds them) the TABLE64 path
+// does the same arithmetic in FP64, culled, and the terms are rounded once.
+// Every term computed in the kernel instead (pair_kernel_f64) stays for larger
+// cutoffs and for counting calls, which report no culled pairs.
+bool f64_table(const lgm_ctx* c) {
+    return c->cfg.precision == LGM_PREC_FP64 && c->d_rtab64 && !c->counting;
+}
+int sum_path(const lgm_ctx* c) { return f64_table(c) ? LGM_PATH_TABLE64 : c->cfg.path; }
+
 // Entries of the table a one-kernel call holds in shared memory.
 int small_table(const lgm_ctx* c, int kind) {
-    if (c->cfg.path == LGM_PATH_TABLE64) return c->rtab_k + 1;
-    if (c->cfg.path == LGM_PATH_TABLE) return (kind == LGM_GAUSS ? c->gtab_k : c->rtab_k) + 1;
+    const int path = sum_path(c);
+    if (path == LGM_PATH_TABLE64) return c->rtab_k + 1;
+    if (path == LGM_PATH_TABLE) return (kind == LGM_GAUSS ? c->gtab_k : c->rtab_k) + 1;
     return kind == LGM_GAUSS ? c->gtab_k + 1 : 0;
 }
 
@@ -854,14 +872,15 @@ SmallFn small_fn(int kind, int path) {
 
 // A call of few sources takes the one-kernel form (lgm_small.cuh): up to
 // kSmallSources of them and kSmallPairs unculled pairs, where the chain's
-// launches cost more than the pairs it culls, with the FP32C precision, no
-// variant forced or tuned for the size, no pair counting, and a table that
-// leaves two CTAs their shared memory.
+// launches cost more than the pairs it culls, with no variant forced or tuned
+// for the size (the FP64 precision has none), no pair counting, and a table
+// that leaves two CTAs their shared memory.
 bool small_call(const lgm_ctx* c, int kind, const Shape& sh, int n, int t) {
-    if (c->cfg.precision == LGM_PREC_FP64 || c->forced_variant >= 0 || c->counting) return false;
+    const bool f64 = c->cfg.precision == LGM_PREC_FP64;
+    if (f64 ? !f64_table(c) : c->forced_variant >= 0 || c->counting) return false;
     if (n < 1 || n > kSmallSources || (long long)n * t * sh.nterms > kSmallPairs) return false;
-    if (c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks))) return false;
-    return small_smem(n, small_table(c, kind), c->cfg.path == LGM_PATH_TABLE64 ? 8 : 4) <= kSmallSmem;
+    if (!f64 && c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks))) return false;
+    return small_smem(n, small_table(c, kind), sum_path(c) == LGM_PATH_TABLE64 ? 8 : 4) <= kSmallSmem;
 }
 
 // flag: null, or the host-visible word the last CTA writes {call, error} to.
@@ -869,6 +888,7 @@ lgm_status launch_small(lgm_ctx* c, int kind, unsigned terms, const int32_t* src
                         int n, const int32_t* tgt, int t, int all_sites, double* out,
                         cudaStream_t st, unsigned long long* flag, unsigned call) {
     const lgm_config& cf = c->cfg;
+    const int path = sum_path(c);
     SmallArgs S{};
     S.src = src; S.q = q; S.n = n;
     S.tgt = all_sites ? nullptr : tgt; S.t = t;
@@ -877,8 +897,8 @@ lgm_status launch_small(lgm_ctx* c, int kind, unsigned terms, const int32_t* src
     S.cell_rank = c->d_cell_rank;
     S.terms = terms;
     S.c2 = (float)(cf.electrostatic_cutoff * cf.electrostatic_cutoff);
-    if (cf.path == LGM_PATH_TABLE64) S.tab64 = kind == LGM_GAUSS ? c->d_gtab64 : c->d_rtab64;
-    else if (cf.path == LGM_PATH_TABLE) S.tab = kind == LGM_GAUSS ? c->d_gtab : c->d_rtab;
+    if (path == LGM_PATH_TABLE64) S.tab64 = kind == LGM_GAUSS ? c->d_gtab64 : c->d_rtab64;
+    else if (path == LGM_PATH_TABLE) S.tab = kind == LGM_GAUSS ? c->d_gtab : c->d_rtab;
     else S.tab = c->d_gtab;
     S.tab_k = small_table(c, kind) - 1;
     S.prefactor = cf.electrostatic_prefactor;
@@ -895,8 +915,8 @@ lgm_status launch_small(lgm_ctx* c, int kind, unsigned terms, const int32_t* src
     const int per = kSmallWarps / S.split;
     const int grid = std::min((segs + per - 1) / per, 4 * c->sm_count);
     if (c->timing) LGM_CUDA(c, cudaEventRecord(c->ev_pair0, st));
-    LGM_CUDA(c, launch_chain(c->overlap, small_fn(kind, cf.path), grid, kSmallThreads,
-                             small_smem(n, S.tab_k + 1, cf.path == LGM_PATH_TABLE64 ? 8 : 4), st, S));
+    LGM_CUDA(c, launch_chain(c->overlap, small_fn(kind, path), grid, kSmallThreads,
+                             small_smem(n, S.tab_k + 1, path == LGM_PATH_TABLE64 ? 8 : 4), st, S));
     if (c->timing) {
         LGM_CUDA(c, cudaEventRecord(c->ev_pair1, st));
         c->timed_pending = true;
@@ -904,7 +924,7 @@ lgm_status launch_small(lgm_ctx* c, int kind, unsigned terms, const int32_t* src
     c->last.ctas = grid;
     c->last.threads = kSmallThreads;
     c->last.targets_per_thread = 1;
-    c->last.variant = kDefaultVariant;
+    c->last.variant = cf.precision == LGM_PREC_FP64 ? -1 : kDefaultVariant;
     c->last.kernel_launches = 1;
     c->last.pairs_tested = (int64_t)popcount3(terms) * t * (int64_t)n;
     c->last.splits = 0;
@@ -940,15 +960,15 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     if (!err_out && small_call(c, kind, sh, n, t))
         return launch_small(c, kind, terms, d_src, d_q, n, d_tgt_site, t, all_sites, d_out, st, nullptr,
                             0);
-    const int v = choose_variant(c, kind, sh);
-    const int fmt =
-        cf.precision == LGM_PREC_FP64 || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
+    const bool f64 = cf.precision == LGM_PREC_FP64, direct = f64 && !f64_table(c);
+    const int v = f64 ? kDefaultVariant : choose_variant(c, kind, sh);
+    const int fmt = direct || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
     lgm_status s;
     if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, fmt, st)) != LGM_OK)
         return s;
     int splits = 1;
     if (c->timing) LGM_CUDA(c, cudaEventRecord(c->ev_pair0, st));
-    if (cf.precision == LGM_PREC_FP64) {
+    if (direct) {
         const double erffactor =
             cf.coulomb_gaussian_sigma > 0 ? 1.0 / (std::sqrt(2.0) * cf.coulomb_gaussian_sigma) : 0.0;
         const int ctas = (sh.t_phys + kF64Threads - 1) / kF64Threads;
@@ -965,7 +985,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         c->last.threads = kF64Threads;
         c->last.targets_per_thread = 1;
     } else {
-        if ((s = launch_pair(c, kind, v, sh, st, &splits)) != LGM_OK) return s;
+        if ((s = launch_pair(c, kind, sum_path(c), v, sh, st, &splits)) != LGM_OK) return s;
     }
     if (c->timing) {
         LGM_CUDA(c, cudaEventRecord(c->ev_pair1, st));
@@ -980,7 +1000,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
                                  c->d_err, err_out));
         c->last.kernel_launches = 5;  // bins (+ scan), scatter, records, pair, finalize
     } else {
-        const Variant& V = kVariants[c->last.variant];
+        const Variant& V = kVariants[v];
         LGM_CUDA(c, launch_chain(c->overlap, finalize_items, (t + 31) / 32, dim3(32, 3), 0, st,
                                  c->d_part, c->d_tile_first, c->d_tile_items, variant_tile(V), t,
                                  sh.t_pad, sh.nterms, cf.electrostatic_prefactor, c->d_perm, d_out,
@@ -988,6 +1008,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         c->last.kernel_launches = 7;  // bins (+ scan), scatter, records, boxes, cull, pair, finalize
     }
     c->bins_clean = true;
+    if (f64) c->last.variant = -1;
     c->last.pairs_tested = (int64_t)sh.nterms * t * (int64_t)n;
     c->last.splits = splits;
     return LGM_OK;
@@ -1221,9 +1242,13 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
                             cudaMemcpyHostToDevice)) != cudaSuccess)
             return bail("cudaMemcpy", e);
     }
-    // FP64 tables of the TABLE64 path: w(k) for every integer r^2 = k <= c^2,
-    // correctly rounded in IEEE double, 0 at k = 0 and k = c^2.
-    if (cf.path == LGM_PATH_TABLE64) {
+    // FP64 tables of the TABLE64 path and of the FP64 precision: w(k) for every
+    // integer r^2 = k <= c^2, correctly rounded in IEEE double, 0 at k = 0 and
+    // k = c^2.
+    const bool tab64 = cf.path == LGM_PATH_TABLE64 ||
+                       (cf.precision == LGM_PREC_FP64 &&
+                        mma_smem_bytes(c2 + 1, 8) <= kF64TableSmem);
+    if (tab64) {
         std::vector<double> rt(c2 + 1, 0.0), gt(c2 + 1, 0.0);
         const double sig = cf.coulomb_gaussian_sigma;
         const double f = sig > 0 ? 1.0 / (std::sqrt(2.0) * sig) : 0.0;
@@ -1271,7 +1296,8 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
                 if (!kernel_of(kVariants[v], fi, c2)) continue;
                 // the table kernels serve only their own path
                 if (fi == 2 && cf.path != LGM_PATH_TABLE) continue;
-                if (fi == 3 && cf.path != LGM_PATH_TABLE64) continue;
+                if (fi == 3 && cf.path != LGM_PATH_TABLE64 && !(tab64 && v == kDefaultVariant))
+                    continue;
                 const size_t smem = variant_smem(kVariants[v], fi, tab_of[fi], c2);
                 if (smem > 48 * 1024) {
                     if (smem > (size_t)smem_optin) {
@@ -1279,9 +1305,15 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
                         lgm_destroy(c);
                         return LGM_ERR_UNSUPPORTED;
                     }
-                    if ((e = cudaFuncSetAttribute(kernel_of(kVariants[v], fi, c2),
+                    // the limit is the function's, not the context's: the
+                    // device's, so that no later context lowers it
+                    cudaFuncAttributes fa;
+                    if ((e = cudaFuncGetAttributes(&fa, kernel_of(kVariants[v], fi, c2))) !=
+                            cudaSuccess ||
+                        (e = cudaFuncSetAttribute(kernel_of(kVariants[v], fi, c2),
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)smem)) != cudaSuccess)
+                                                  smem_optin - (int)fa.sharedSizeBytes)) !=
+                            cudaSuccess)
                         return bail("cudaFuncSetAttribute", e);
                 }
                 int bps = 0;
@@ -1293,7 +1325,7 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
             }
     }
     for (int k : {LGM_POINT, LGM_GAUSS})
-        if ((e = cudaFuncSetAttribute(small_fn(k, cf.path), cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if ((e = cudaFuncSetAttribute(small_fn(k, tab64 ? (int)LGM_PATH_TABLE64 : cf.path), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kSmallSmem)) != cudaSuccess)
             return bail("cudaFuncSetAttribute", e);
     *out = c;
@@ -1440,11 +1472,11 @@ lgm_status lgm_autotune(lgm_ctx* c, lgm_kind kind, uint32_t terms, int32_t n, in
     for (int v = 0; v < kNumVariants; ++v) {
         if (c->cfg.path == LGM_PATH_TABLE64 && !kVariants[v].cull) continue;
         int splits;
-        if ((s = launch_pair(c, kind, v, sh, st, &splits)) != LGM_OK) break;  // warm
+        if ((s = launch_pair(c, kind, c->cfg.path, v, sh, st, &splits)) != LGM_OK) break;  // warm
         float ms[3];
         for (int r = 0; r < 3; ++r) {
             cudaEventRecord(e0, st);
-            if ((s = launch_pair(c, kind, v, sh, st, &splits)) != LGM_OK) break;
+            if ((s = launch_pair(c, kind, c->cfg.path, v, sh, st, &splits)) != LGM_OK) break;
             cudaEventRecord(e1, st);
             cudaEventSynchronize(e1);
             cudaEventElapsedTime(&ms[r], e0, e1);
