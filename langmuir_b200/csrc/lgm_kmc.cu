@@ -565,10 +565,15 @@ __device__ __forceinline__ void decide_body(const Dev& D, const int i) {
 // faster than 256 for a single replica (256x256x16, 20,922 carriers: step
 // 0.646 -> 0.620 ms) and for a batch of 512 uneven replicas (2.27 -> 2.20 ms).
 constexpr int kGuardThreads = 1024;
-// Each queued decision's source range is cut into this many splits, one
-// block each; the block that completes a decision last adds the splits'
-// partials in split order (a fixed order) and decides.
+// Each queued decision's source range is cut into splits of at least
+// kGuardSplitSources, kGuardSplits at most, one block each; the block that
+// completes a decision last adds the splits' partials in split order (a fixed
+// order) and decides.  A split costs its block two barriers and an atomic
+// whatever its length, so 16 for every replica were dear for small ones (512
+// uneven replicas, 100 steps and the read-out: 183.3 ms, as here 180.4; 64:
+// 35.4 and 33.8).
 constexpr int kGuardSplits = 16;
+constexpr int kGuardSplitSources = 1024;
 // Blocks per replica of the batched guard: flagged decisions of one replica
 // are spread over them (a replica with M charges flags ~1e-3 M per step).
 constexpr int kGuardBlocksPerReplica = 48;
@@ -576,8 +581,13 @@ constexpr int kGuardBlocksPerReplica = 48;
 // block with nothing to do costs its launch and retirement, so they are
 // small; a replica gets one block per 512 charges of capacity.
 constexpr int kGuardThreadsBatch = 256;
-// Indices per thread of the batched element-wise kernels (see LGM_BATCH_LOOP).
-constexpr int kItemsPerThread = 4;
+// Indices per thread of the batched element-wise kernels (see LGM_BATCH_LOOP):
+// their time is a chain of dependent loads per index, so two while the batch's
+// blocks fill the chip many times over, else one (100 steps and the read-out
+// at 1, 2 and 4 indices: 512 uneven replicas 184, 179 and 180 ms, 64 30.5, 31.1
+// and 33.8; at 1 and 2: 16 replicas 13.0 and 14.6).
+constexpr int kItemsPerThread = 2;
+constexpr int kBlocksPerSmOfOne = 8;  // one index a thread up to so many blocks an SM
 
 // FP64 potentials at two sites in one pass over the sources (the guard's
 // re-evaluation): the same cutoff and image rules as the pair kernel, terms
@@ -640,27 +650,28 @@ __device__ __forceinline__ void guard_body(const Dev& D, const int block, const 
     const int nflag = D.cnt[I_NFLAG];
     const uint32_t step = (uint32_t)D.cnt[I_STEP];
     const int n = ne + nh + (D.dq != 0 ? D.nd : 0);
-    for (int w = block; w < nflag * kGuardSplits; w += nblocks) {
-        const int q_i = w / kGuardSplits, sp = w - q_i * kGuardSplits;
+    const int splits = min(kGuardSplits, max(1, n / kGuardSplitSources));
+    for (int w = block; w < nflag * splits; w += nblocks) {
+        const int q_i = w / splits, sp = w - q_i * splits;
         const int i = D.flagged[q_i];
         const bool e = i < ne;
         const int k = e ? i : i - ne;
         const int site = e ? D.e_site[k] : D.h_site[k];
         const int f = e ? D.e_f[k] : D.h_f[k];
         const double q = e ? -1.0 : 1.0;
-        const int j0 = (int)((long long)sp * n / kGuardSplits);
-        const int j1 = (int)((long long)(sp + 1) * n / kGuardSplits);
+        const int j0 = (int)((long long)sp * n / splits);
+        const int j1 = (int)((long long)(sp + 1) * n / splits);
         const double2 part = fp64_potential2(D, ne, nh, site, f, j0, j1, red);
         if (threadIdx.x == 0) {
             D.gpart[(size_t)q_i * kGuardSplits + sp] = part;
             __threadfence();
-            s_last = atomicAdd(&D.gdone[q_i], 1) == kGuardSplits - 1;
+            s_last = atomicAdd(&D.gdone[q_i], 1) == splits - 1;
         }
         __syncthreads();
         if (s_last && threadIdx.x == 0) {
             __threadfence();
             double2 t = make_double2(0.0, 0.0);
-            for (int u = 0; u < kGuardSplits; ++u) {  // split order
+            for (int u = 0; u < splits; ++u) {  // split order
                 const double2 p = __ldcg(&D.gpart[(size_t)q_i * kGuardSplits + u]);
                 t.x += p.x;
                 t.y += p.y;
@@ -1206,7 +1217,7 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact_inject(Dev D) {
 // map[b].y of map[b].z blocks, over indices [0, map[b].w) of that replica with
 // a block-uniform stride (every block lies inside one replica, so warp-level
 // sums stay within a replica, and every thread of a block runs the same number
-// of iterations).  A replica gets one block per kItemsPerThread * 256 indices
+// of iterations).  A replica gets one block per 256 or kItemsPerThread * 256 indices
 // of its capacity, so small replicas in a big batch cost few idle blocks.
 #define LGM_BATCH_LOOP(CALL)                                                          \
     const int4 m = map[blockIdx.x];                                                   \
@@ -3021,8 +3032,11 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
         cargs[r] = cull_args(D);
     }
     std::vector<int4> car, pack, fin, guard, bins;
-    auto add = [](std::vector<int4>& v, int r, int bound) {
-        const int nb = std::max(1, (bound + kItemsPerThread * 256 - 1) / (kItemsPerThread * 256));
+    long long blocks = 0;  // at one index a thread, of the carriers
+    for (int r : b->classic) blocks += (b->hD[r].cap_e + b->hD[r].cap_h + 255) / 256;
+    const int per = blocks <= (long long)kBlocksPerSmOfOne * b->reps[0]->sm_count ? 1 : kItemsPerThread;
+    auto add = [per](std::vector<int4>& v, int r, int bound) {
+        const int nb = std::max(1, (bound + per * 256 - 1) / (per * 256));
         for (int i = 0; i < nb; ++i) v.push_back(make_int4(r, i, nb, bound));
     };
     int max_cap = 1;
