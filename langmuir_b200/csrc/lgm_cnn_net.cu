@@ -161,7 +161,14 @@ conv1_planes(const uint32_t* __restrict__ x, const float* __restrict__ w,
                     float d[2][4];
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
-                        mma16816(d[s], a[j], bw[s][n][0], bw[s][n][1], bv[n][0], bv[n][1]);
+                        mma16816(d[s], a[j], bw[s][n][0], bw[s][n][1], 0.f, 0.f);
+#pragma unroll
+                        for (int v = 0; v < 4; v += 2) {  // the bias in FP32, after the sum
+                            const float2 e = __fadd2_rn(make_float2(d[s][v], d[s][v + 1]),
+                                                        make_float2(bv[n][0], bv[n][1]));
+                            d[s][v] = e.x;
+                            d[s][v + 1] = e.y;
+                        }
 #pragma unroll
                         for (int v = 0; v < 4; ++v) {
                             d[s][v] = fmaxf(d[s][v], 0.f);
@@ -663,10 +670,26 @@ head_fwd(const uint4* __restrict__ a4, int HW, const float* __restrict__ w1,
          const float* __restrict__ b1, const float* __restrict__ w2, const float* __restrict__ b2,
          uint16_t* __restrict__ g16, uint16_t* __restrict__ h16, float* __restrict__ y) {
     __shared__ __align__(16) unsigned char s_a[PL * GAP_STRIDE];
-    __shared__ float s_g[CH], s_h[HID], s_w1[HID * (CH + 1)], s_w2[OUT * HID];
+    __shared__ __align__(4) uint16_t s_g[CH], s_h[HID];
     const int b = blockIdx.x, tid = threadIdx.x;
-    for (int i = tid; i < HID * CH; i += 256) s_w1[(i / CH) * (CH + 1) + i % CH] = bf(to_bf(w1[i]));
-    if (tid < OUT * HID) s_w2[tid] = bf(to_bf(w2[tid]));
+    // The products on the tensor cores, K in steps of 16, the image in row 0 of
+    // 16; a warp takes eight hidden units.
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    uint32_t f1[CH / 16][2], f2[HID / 16][2];
+#pragma unroll
+    for (int k = 0; k < CH / 16; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float* p = w1 + (8 * warp + g) * CH + 16 * k + 8 * h + 2 * t;
+            f1[k][h] = pack2(p[0], p[1]);
+        }
+#pragma unroll
+    for (int k = 0; k < HID / 16; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float* p = w2 + g * HID + 16 * k + 8 * h + 2 * t;
+            f2[k][h] = warp == 0 && g < OUT ? pack2(p[0], p[1]) : 0u;
+        }
     lgm::pdl_wait();
     lgm::pdl_trigger();
     const uint4* img = a4 + (size_t)b * PL * HW;
@@ -686,26 +709,42 @@ head_fwd(const uint4* __restrict__ a4, int HW, const float* __restrict__ w1,
     }
     if (tid < CH) {
         const uint16_t v = to_bf(s / (float)HW);
-        s_g[tid] = bf(v);
+        s_g[tid] = v;
         g16[(size_t)b * CH + tid] = v;
     }
     __syncthreads();
-    if (tid < HID) {
-        float h = 0.f;
+    // row 0 of A: thread t of the first four holds k = 2t, 2t+1, 2t+8, 2t+9
+    auto row0 = [&](const uint16_t* src, int k, uint32_t (&a)[4]) {
+        a[0] = g == 0 ? *reinterpret_cast<const uint32_t*>(src + 16 * k + 2 * t) : 0u;
+        a[2] = g == 0 ? *reinterpret_cast<const uint32_t*>(src + 16 * k + 8 + 2 * t) : 0u;
+        a[1] = a[3] = 0u;
+    };
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int c = 0; c < CH; ++c) h = fmaf(s_g[c], s_w1[tid * (CH + 1) + c], h);
-        h = fmaxf(h + b1[tid], 0.f);
-        const uint16_t v = to_bf(h);
-        s_h[tid] = bf(v);
-        h16[(size_t)b * HID + tid] = v;
+    for (int k = 0; k < CH / 16; ++k) {
+        uint32_t a[4];
+        row0(s_g, k, a);
+        mma16816(c, a, f1[k][0], f1[k][1]);
     }
+    if (g == 0)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int n = 8 * warp + 2 * t + i;
+            const uint16_t v = to_bf(fmaxf(c[i] + b1[n], 0.f));
+            s_h[n] = v;
+            h16[(size_t)b * HID + n] = v;
+        }
     __syncthreads();
-    if (tid < OUT) {
-        float o = 0.f;
+    if (warp != 0) return;
+    c[0] = c[1] = c[2] = c[3] = 0.f;
 #pragma unroll
-        for (int j = 0; j < HID; ++j) o = fmaf(s_h[j], s_w2[tid * HID + j], o);
-        y[(size_t)b * OUT + tid] = o + b2[tid];
+    for (int k = 0; k < HID / 16; ++k) {
+        uint32_t a[4];
+        row0(s_h, k, a);
+        mma16816(c, a, f2[k][0], f2[k][1]);
     }
+    if (lane == 0)
+        for (int i = 0; i < OUT; ++i) y[(size_t)b * OUT + i] = c[i] + b2[i];
 }
 
 // One block per image: the gradient through the head down to a4's ReLU,

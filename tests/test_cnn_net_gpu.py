@@ -45,3 +45,31 @@ def test_native_network_matches_oracle(B, H, W):
         again, _ = S.network_forward(S.phases_to_input(ph),
                                      [torch.as_tensor(p).cuda() for p in P], keep=False)
     np.testing.assert_array_equal(again.cpu().numpy(), yg)
+
+
+@pytest.mark.parametrize("n,H,W,seed", [(256, 128, 128, 1), (256, 128, 128, 2), (33, 64, 256, 3),
+                                        (1, 64, 128, 4)])
+def test_native_forward_has_the_layers_bits(n, H, W, seed):
+    """The native forward pass adds in the per-layer kernels' order, so no BF16
+    activation rounds the other way: the outputs are equal, not close."""
+    import torch
+    from langmuir_b200 import surrogate as S
+    ph, _, _ = S.grf_morphologies(n, size=max(H, W), seed=seed)
+    x = S.phases_to_input(ph[:, :H, :W].contiguous(), ramp=0.5)
+    params = S.init_params(seed)
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    with torch.no_grad():
+        for i in (1, 3, 5, 7, 9, 11):
+            params[i].copy_(torch.randn(params[i].shape, generator=g, device="cuda") * 0.1)
+        y, _ = S.network_forward(x, params, keep=False)
+        c1w, c1b, c2w, c2b, c3w, c3b, c4w, c4b, f1w, f1b, f2w, f2b = params
+        p = x
+        for k, (w, b, cin) in enumerate([(c1w, c1b, 1), (c2w, c2b, S.CH), (c3w, c3b, S.CH)]):
+            _, p = S.conv3x3(p, S.conv_weights_bf16(w, cin), b, H >> k, W >> k, keep_act=False)
+        a4, _ = S.conv3x3(p, S.conv_weights_bf16(c4w, S.CH), c4b, H >> 3, W >> 3, pool=False)
+        _, g16 = S.gap_fwd(a4)
+        hid, out = S.HIDDEN, S.OUTPUTS
+        h = S.to_bf16(S.gemm(g16, S.CH, 1, f1w.to(torch.bfloat16), 1, S.CH, n, hid, S.CH, bias=f1b,
+                             relu=True))
+        want = S.gemm(h, hid, 1, f2w.to(torch.bfloat16), 1, hid, n, out, hid, bias=f2b)
+    np.testing.assert_array_equal(y.cpu().numpy(), want.cpu().numpy())
