@@ -87,12 +87,19 @@ __device__ __forceinline__ uint32_t half_mask(uint32_t m) { return (m & 0x10001u
 // without shuffles; with the columns permuted a thread holds channels 8t ..
 // 8t+7 and stores one 16-byte vector.  The input comes straight from L1, two
 // words and a funnel shift per fragment.
-// Bound: HBM (the pooled output) and the ReLU/pool arithmetic, about 85
-// instructions per 1024 values.  1024 images of 128x128: the shared-memory
-// tile of conv1_fwd took 242 us.
+// A row is a few steps long, so the first words of the warp's next row are
+// loaded over the last step of this one, and the row index is stepped without a
+// division.  Two blocks an SM hold that without spills (128 registers): 4096
+// images of 128x128, four networks, 4.92 ms plain with three blocks, 4.79 so.
+// (At 80 registers for three blocks it spilled and lost 2%; with 8 pixels in
+// flight instead of 16 half the gain was left.)
+// Bound: the ReLU/pool arithmetic, about 100 instructions per 1024 values (ALU
+// pipe half busy), then HBM (the pooled output of 1024 images, 41 us).  The
+// shared-memory tile of conv1_fwd took 242 us for 1024 images, the plain loop 120.
 constexpr int C1_WARPS = 8;
+constexpr int C1_CTAS = 2;  // an SM
 template <bool MASK>
-__global__ void __launch_bounds__(C1_WARPS * 32, 3)
+__global__ void __launch_bounds__(C1_WARPS * 32, C1_CTAS)
 conv1_planes(const uint32_t* __restrict__ x, const float* __restrict__ w,
              const float* __restrict__ bias, uint4* __restrict__ pooled,
              uint32_t* __restrict__ mask, int B, int H, int W) {
@@ -117,42 +124,61 @@ conv1_planes(const uint32_t* __restrict__ x, const float* __restrict__ w,
     }
     const int H2 = H / 2, W2 = W / 2;  // W2 is also the words of an input row
     const int i0 = g - 1 + (t & 1);    // this thread's first word
-    const long long rows = (long long)B * H2;
-    for (long long r = (long long)blockIdx.x * C1_WARPS + (threadIdx.x >> 5); r < rows;
-         r += (long long)gridDim.x * C1_WARPS) {
-        const int b = (int)(r / H2), py = (int)(r - (long long)b * H2);
-        const uint32_t* img = x + (size_t)b * H * W2;
-        // The rows of this thread's four fragments, from its first word on.
-        // Outside the image, and in the zero slots, a row inside is read and
-        // masked out.
+    // pooled rows of the batch (a row's output is 1 KB or more, so 31 bits hold them)
+    const int rows = B * H2, stride = (int)gridDim.x * C1_WARPS;
+    const int sb = stride / H2, sy = stride - sb * H2;  // a stride in images and rows
+    int r = (int)blockIdx.x * C1_WARPS + (threadIdx.x >> 5);
+    if (r >= rows) return;
+    int b = r / H2, py = r - b * H2;
+    // The rows of this thread's four fragments, from its first word on.  Outside
+    // the image, and in the zero slots, a row inside is read and masked out.
+    const uint32_t* rp[4];
+    uint32_t keep[4];
+    auto set_row = [&] {
+        const uint32_t* img = x + (size_t)b * H * W2 + i0;
         const int ya = 2 * py - 1 + (t >> 1), yd = 2 * py + 2;
-        const uint32_t keep[4] = {ya >= 0 ? ~0u : 0u, ~0u, t < 2 ? ~0u : 0u,
-                                  t < 2 && yd < H ? ~0u : 0u};
-        const uint32_t* rp[4] = {img + (long long)max(ya, 0) * W2 + i0,
-                                 img + (long long)(ya + 1) * W2 + i0,
-                                 img + (long long)(2 * py + 1) * W2 + i0,
-                                 img + (long long)min(yd, H - 1) * W2 + i0};
+        keep[0] = ya >= 0 ? ~0u : 0u;
+        keep[1] = ~0u;
+        keep[2] = t < 2 ? ~0u : 0u;
+        keep[3] = t < 2 && yd < H ? ~0u : 0u;
+        rp[0] = img + max(ya, 0) * W2;
+        rp[1] = img + (ya + 1) * W2;
+        rp[2] = img + (2 * py + 1) * W2;
+        rp[3] = img + min(yd, H - 1) * W2;
+    };
+    // words i, i+1 hold pixels 2i+1, 2i+2; a row's ends have none outside
+    uint32_t lo[2][4], hi[2][4];
+    auto load = [&](int p0) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                lo[j][k] = j == 0 && p0 == 0 && i0 < 0 ? 0u : rp[k][p0 + 8 * j];
+                hi[j][k] = j == 1 && p0 + 16 == W2 && i0 == 7 ? 0u : rp[k][p0 + 8 * j + 1];
+            }
+    };
+    set_row();
+    load(0);
+    for (;;) {
         uint4* prow = pooled + (((size_t)b * PL + t) * H2 + py) * W2 + g;
         uint32_t* mrow = MASK ? mask + (((size_t)b * H2 + py) * W2 + g) * 4 + t : nullptr;
-        // words i, i+1 hold pixels 2i+1, 2i+2; a row's ends have none outside
-        uint32_t lo[2][4], hi[2][4];
-        auto load = [&](int p0) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    lo[j][k] = j == 0 && p0 == 0 && i0 < 0 ? 0u : rp[k][p0 + 8 * j];
-                    hi[j][k] = j == 1 && p0 + 16 == W2 && i0 == 7 ? 0u : rp[k][p0 + 8 * j + 1];
-                }
-        };
-        load(0);
         for (int p0 = 0; p0 < W2; p0 += 16) {
             uint32_t a[2][4];
 #pragma unroll
             for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) a[j][k] = __funnelshift_r(lo[j][k], hi[j][k], 16) & keep[k];
-            if (p0 + 16 < W2) load(p0 + 16);  // in flight over this step's arithmetic
+            // the next words are in flight over this step's arithmetic, past the
+            // row's end those of the warp's next row
+            if (p0 + 16 < W2) {
+                load(p0 + 16);
+            } else if ((r += stride) < rows) {
+                b += sb;
+                py += sy;
+                if (py >= H2) { py -= H2; ++b; }
+                set_row();
+                load(0);
+            }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 uint32_t out[4], sub[4] = {0u, 0u, 0u, 0u};
@@ -193,6 +219,7 @@ conv1_planes(const uint32_t* __restrict__ x, const float* __restrict__ w,
                 prow[p0 + 8 * j] = make_uint4(out[0], out[1], out[2], out[3]);
             }
         }
+        if (r >= rows) return;
     }
 }
 
@@ -1039,7 +1066,7 @@ lgm_status lgm_cnn_net_forward(const void* x, const float* const* params, void* 
     const Saved L = saved_layout(B, H, W, keep != 0);
     char* w = (char*)saved;
     const int grid1 = (int)std::min<long long>(((long long)B * (H / 2) + C1_WARPS - 1) / C1_WARPS,
-                                               d.sms * 3ll);
+                                               (long long)d.sms * C1_CTAS);
     if (keep)
         conv1_planes<true><<<grid1, C1_WARPS * 32, 0, st>>>((const uint32_t*)x, params[0], params[1],
                                                             (uint4*)(w + L.p1), (uint32_t*)(w + L.m1),
