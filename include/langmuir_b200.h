@@ -249,7 +249,8 @@ lgm_status lgm_set_counting(lgm_ctx* ctx, int32_t enable);
  * charges of the given size (n sources, t targets, `terms`) with CUDA events,
  * remembers the fastest for that size bucket (half-octaves of targets and
  * source chunks) on this context, and reports it; calls in an untuned bucket
- * use variant 0.  It allocates, so call it before any stream capture. */
+ * use the last variant, or one kernel when they have few sources (up to 2048,
+ * and 2^25 pairs).  It allocates, so call it before any stream capture. */
 lgm_status lgm_autotune(lgm_ctx* ctx, lgm_kind kind, uint32_t terms, int32_t n, int32_t t,
                         int32_t* chosen);
 /* Force a variant (0 .. lgm_variant_count()-1) for every call, -1 = automatic. */
@@ -278,6 +279,8 @@ lgm_status lgm_variant_info(int32_t variant, int32_t* threads, int32_t* target_p
  * of lgm_variant_info counts the target warps' threads only. */
 #define LGM_VARIANT_WARP_SPECIALISED 4
 lgm_status lgm_variant_flags(int32_t variant, int32_t* flags);
+/* The last variant, the default, is culled too: r^2 from the tensor cores, each
+ * warp on items of its own 32 targets; its `target_pairs` reads 1. */
 /* Culled variants: source chunks per work item (at least; more when a
  * tile's live chunks exceed 32 items) and, warp-specialised, the stages of
  * the copy ring (0 otherwise); both 0 for the other variants. */

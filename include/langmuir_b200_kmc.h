@@ -214,7 +214,9 @@ lgm_status lgm_kmc_last_outcomes(lgm_kmc* k, int32_t* outcome, double* de, int32
  * voltages and traps may all differ; the interaction kind must not), advanced
  * together.  Replica i uses the random stream of a single replica with id
  * replica0 + i, so its trajectory equals that of
- * lgm_kmc_create(&params[i], device, replica0 + i).
+ * lgm_kmc_create(&params[i], device, replica0 + i).  (A small replica of
+ * lgm_kmc_create takes the fused form as well: room for at most 512 charges
+ * and 2^18 carriers x sources x terms.)
  * Two step forms share the batch:
  *  - fused: each replica runs the whole step inside one block, many steps
  *    per launch;
