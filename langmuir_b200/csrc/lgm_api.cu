@@ -1163,11 +1163,9 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
         return LGM_ERR_NO_DEVICE;
     }
     // attribute reads: cudaGetDeviceProperties takes 2.5 ms and more
-    int cc_major = 0, n_sms = 0, smem_optin = 0;
+    int cc_major = 0, n_sms = 0;
     if ((e = cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) !=
-            cudaSuccess) {
+        (e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) {
         g_create_error = std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e);
         return LGM_ERR_NO_DEVICE;
     }
@@ -1299,22 +1297,13 @@ lgm_status lgm_create(const lgm_config* cfg, int32_t device, lgm_ctx** out) {
                 if (fi == 3 && cf.path != LGM_PATH_TABLE64 && !(tab64 && v == kDefaultVariant))
                     continue;
                 const size_t smem = variant_smem(kVariants[v], fi, tab_of[fi], c2);
-                if (smem > 48 * 1024) {
-                    if (smem > (size_t)smem_optin) {
-                        g_create_error = "cutoff too large for the shared-memory tables";
-                        lgm_destroy(c);
-                        return LGM_ERR_UNSUPPORTED;
-                    }
-                    // the limit is the function's, not the context's: the
-                    // device's, so that no later context lowers it
-                    cudaFuncAttributes fa;
-                    if ((e = cudaFuncGetAttributes(&fa, kernel_of(kVariants[v], fi, c2))) !=
-                            cudaSuccess ||
-                        (e = cudaFuncSetAttribute(kernel_of(kVariants[v], fi, c2),
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  smem_optin - (int)fa.sharedSizeBytes)) !=
-                            cudaSuccess)
-                        return bail("cudaFuncSetAttribute", e);
+                bool fits = false;
+                if ((e = allow_smem(kernel_of(kVariants[v], fi, c2), smem, &fits)) != cudaSuccess)
+                    return bail("shared-memory limit", e);
+                if (!fits) {
+                    g_create_error = "cutoff too large for the shared-memory tables";
+                    lgm_destroy(c);
+                    return LGM_ERR_UNSUPPORTED;
                 }
                 int bps = 0;
                 if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(

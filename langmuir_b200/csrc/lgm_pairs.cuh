@@ -84,6 +84,25 @@ inline size_t pair_smem_bytes64(int tab_k) {
     return 2 * pair_stage_bytes() + 16 + (size_t)(tab_k + 1) * sizeof(double) + 16;
 }
 
+// Lets kernel `fn` launch with `bytes` of dynamic shared memory.  A block gets 48 KB
+// unasked, its static part included.  The limit belongs to the function, for every
+// context, replica and batch of the process: it goes up to all the device has, so
+// that none of them lowers it under another.  *fits: static and dynamic part are
+// within that.
+inline cudaError_t allow_smem(const void* fn, size_t bytes, bool* fits = nullptr) {
+    cudaFuncAttributes fa;
+    int dev = 0, most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e != cudaSuccess) return e;
+    if (fits) *fits = fa.sharedSizeBytes + bytes <= (size_t)most;
+    if (fa.sharedSizeBytes + bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                most - (int)fa.sharedSizeBytes);
+}
+
 // KIND 0 point, 1 gauss.  PATH 0 MUFU rsqrt, 1 shared-memory table of w(k)
 // for every integer r^2 = k (entries 0 and c^2 are 0).  NT threads, RP target
 // pairs per thread, SUB sources per FP32 run (SUB divides CH).

@@ -1,0 +1,59 @@
+"""Tables that bring a kernel's static and dynamic shared memory to either side of
+the 48 KB a block gets unasked: FP64 entries at cutoffs 74 to 79, FP32 ones at 105
+to 111.  Each kind of table in a process of its own, small tables first, since a
+limit once raised stays raised for the process.
+
+Tolerance: an FP32 weight is rounded once and added in runs of 16, so a sum is
+within 17 2^-24 of its terms' magnitudes; in FP64 (test_fp64_sums_gpu) within
+2 (n + 4) 2^-53."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+DIMS = (61, 47, 5)
+N_SRC = 3000  # too many for the one-kernel form
+
+CHILD = """
+import sys
+import numpy as np
+import langmuir_b200 as L
+z = np.load(sys.argv[1])
+keys = dict(fp64=dict(precision=L.PREC_FP64), table64=dict(path=2), table=dict(path=1))[sys.argv[2]]
+out = {}
+for c in map(int, sys.argv[3:]):
+    with L.Coulomb(*map(int, z["dims"]), cutoff=c, **keys) as ctx:
+        out[str(c)] = ctx.potentials(z["src"], z["q"], z["tgt"], L.POINT, 7)
+        assert ctx.last_launch()["kernel_launches"] == 7
+        if sys.argv[2] != "fp64":
+            ctx.autotune(len(z["src"]), len(z["tgt"]), L.POINT, 7)
+np.savez(sys.argv[1] + ".out.npz", **out)
+"""
+
+
+@pytest.mark.parametrize("table,cutoffs", [("fp64", (74, 75, 78, 79)), ("table64", (74, 75, 78, 79)),
+                                           ("table", (105, 106, 110, 111))])
+def test_tables_around_the_default_limit(oracle_mod, tmp_path, table, cutoffs):
+    rng = np.random.default_rng(5)
+    V = DIMS[0] * DIMS[1] * DIMS[2]
+    src = rng.choice(V, N_SRC, replace=False).astype(np.int32)
+    q = rng.choice([-2, -1, 1, 3], N_SRC).astype(np.int32)
+    tgt = rng.integers(0, V, 501).astype(np.int32)
+    f = str(tmp_path / "in.npz")
+    np.savez(f, dims=DIMS, src=src, q=q, tgt=tgt)
+    r = subprocess.run([sys.executable, "-c", CHILD, f, table, *map(str, cutoffs)],
+                       capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-800:]
+    got = np.load(f + ".out.npz")
+    rel = 17 * 2.0 ** -24 if table == "table" else 2 * (N_SRC + 4) * 2.0 ** -53
+    for c in cutoffs:
+        orc = oracle_mod.Oracle(*DIMS, cutoff=c)
+        want = orc.potentials(src, q, tgt, terms=7)
+        direct = orc.potentials(src, np.abs(q), tgt, terms=1)
+        norm = 2 * direct - orc.potentials(src, np.abs(q), tgt, terms=7)
+        assert np.all(np.abs(got[str(c)] - want) <= rel * norm)
