@@ -2419,12 +2419,13 @@ static lgm_status kmc_create_impl(const lgm_params* pin, int32_t device, uint32_
             return bail(LGM_ERR_CUDA, "table upload");
         D.gtab = k->gtab;
         D.gtab_k = kmax;
-        for (int sorted = 0; sorted < 2; ++sorted)
-            cudaFuncSetAttribute(kmc_pair(1, sorted), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)pair_smem_bytes(kmax));
-        cudaFuncSetAttribute(kmc_pair_culled(1, D.cutoff2),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kmc_culled_smem(D.cutoff2, kmax));
+        cudaError_t e = cudaSuccess;
+        for (int sorted = 0; sorted < 2 && e == cudaSuccess; ++sorted)
+            e = allow_smem(reinterpret_cast<const void*>(kmc_pair(1, sorted)), pair_smem_bytes(kmax));
+        if (e == cudaSuccess)
+            e = allow_smem(reinterpret_cast<const void*>(kmc_pair_culled(1, D.cutoff2)),
+                           kmc_culled_smem(D.cutoff2, kmax));
+        if (e != cudaSuccess) return bail(LGM_ERR_CUDA, "shared memory of the pair sums");
     }
     cudaMemcpy(crank_d, crank.data(), sizeof(int32_t) * crank.size(), cudaMemcpyHostToDevice);
     D.cell_rank = crank_d;
@@ -3130,11 +3131,9 @@ lgm_status lgm_kmc_batch_create(const lgm_params* params, int32_t count, int32_t
         cudaMalloc(&b->d_pargs, sizeof(PairArgs) * count) != cudaSuccess)
         return bail(LGM_ERR_CUDA, "descriptors");
     if (b->gauss) {
-        cudaFuncSetAttribute(kBatchVariants[0].fn[1], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)batch_smem(b));
         for (const BatchVariant& BV : kBatchVariants)
-            cudaFuncSetAttribute(BV.fn[1], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)batch_smem(b));
+            if (allow_smem(reinterpret_cast<const void*>(BV.fn[1]), batch_smem(b)) != cudaSuccess)
+                return bail(LGM_ERR_CUDA, "shared memory of the pair sums");
     }
     if (cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||

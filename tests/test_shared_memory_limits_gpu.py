@@ -57,3 +57,44 @@ def test_tables_around_the_default_limit(oracle_mod, tmp_path, table, cutoffs):
         direct = orc.potentials(src, np.abs(q), tgt, terms=1)
         norm = 2 * direct - orc.potentials(src, np.abs(q), tgt, terms=7)
         assert np.all(np.abs(got[str(c)] - want) <= rel * norm)
+
+
+def gaussian_params(L, cutoff, sigma):
+    return L.Params.default(grid_x=64, grid_y=64, grid_z=8, electron_percentage=0.03,
+                            hole_percentage=0.03, seed_charges=1.0, coulomb_carriers=1,
+                            electrostatic_cutoff=cutoff, coulomb_gaussian_sigma=sigma,
+                            voltage_right=1.0, h_source_r_rate=0.9, h_drain_l_rate=0.9,
+                            random_seed=3)
+
+
+@pytest.mark.parametrize("first,then", [((50, 1.0), (20, 1.0)), ((30, 3.0), (30, 1.0))])
+def test_a_gaussian_replica_leaves_an_older_one_its_tables(oracle_mod, first, then):
+    """The older replica runs last, and steps as the oracle does."""
+    import langmuir_b200 as L
+    from oracle.kmc_setup import independent_world, oracle_for
+    p = gaussian_params(L, *first)
+    with L.KMC(p, replica=2) as a, L.KMC(gaussian_params(L, *then)) as b:
+        b.run(2)
+        st = a.stats()
+        e0, h0 = a.carriers()
+        orc = oracle_for(oracle_mod, p, independent_world(p, 2), e0, h0, st["max_electrons"],
+                         st["max_holes"], replica=2)
+        a.run(3)
+        for _ in range(3):
+            orc.step()
+        for got, want in zip(a.carriers(), orc.carriers()):
+            np.testing.assert_array_equal(got, want)
+
+
+def test_a_gaussian_batch_leaves_an_older_one_its_tables():
+    import langmuir_b200 as L
+    out = []
+    for between in (False, True):
+        with L.KMCBatch([gaussian_params(L, 60, 8.0)], fused_max_charges=1) as a:
+            if between:
+                with L.KMCBatch([gaussian_params(L, 20, 1.0)], fused_max_charges=1) as b:
+                    b.run(2)
+            a.run(3)
+            out.append(a.replica(0).carriers())
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
