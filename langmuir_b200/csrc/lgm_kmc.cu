@@ -923,8 +923,10 @@ __device__ void block_try_inject(const Dev& D, InjectState& S, int s, uint32_t s
         S.u = unit_double(r.w[1], r.w[2]);
     }
     __syncthreads();
-    if (!S.valid) return;
+    const bool valid = S.valid;
     const int site = S.site;
+    __syncthreads();  // every thread has read them before a later try writes them
+    if (!valid) return;
     double de = 0.0;
     if (D.src_metro) {
         double p2 = D.pot[site];

@@ -115,3 +115,24 @@ def test_small_single_replicas_match_oracle(oracle_mod, cap, keys):
             np.testing.assert_array_equal(e, e_o)
             np.testing.assert_array_equal(h, h_o)
             np.testing.assert_array_equal(np.array(k.stats()["counters"], np.uint64), orc.counters)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("coulomb", [0, 1])
+def test_rejected_source_tries_match_oracle(oracle_mod, coulomb):
+    """Metropolis sources on faces that are nearly always full: tries that find
+    their site taken follow one another without a pair sum between them."""
+    p = params(grid_x=4, grid_y=3, grid_z=2, electron_percentage=0.6, hole_percentage=0.6,
+               seed_charges=1.0, h_source_l_rate=1.0, h_source_r_rate=1.0, source_metropolis=1,
+               source_coulomb=coulomb)
+    with L.KMC(p, replica=5) as k:
+        st = k.stats()
+        e0, h0 = k.carriers()
+        orc = oracle_for(oracle_mod, p, independent_world(p, 5), e0, h0, st["max_electrons"],
+                         st["max_holes"], replica=5)
+        for _ in range(200):
+            orc.step()
+        k.run(200)
+        for got, want in zip(k.carriers(), orc.carriers()):
+            np.testing.assert_array_equal(got, want)
+        np.testing.assert_array_equal(np.array(k.stats()["counters"], np.uint64), orc.counters)
