@@ -83,8 +83,8 @@ lgm_status lgm_cnn_to_bf16(const float* in, void* out, int32_t n, const float* r
 /* The whole network in one call, on kernels that share one internal layout
  * (FP32 masters in; the BF16 roundings of the layer-by-layer kernels).
  * params[12]: c1w [32][9], c1b, c2w [32][288], c2b, c3w, c3b, c4w, c4b,
- * f1w [64][32], f1b, f2w [2][64], f2b.  x: [B][H][W] BF16, H % 16 == 0,
- * W % 64 == 0; y: [B][2] FP32.  saved: device memory of lgm_cnn_net_bytes(B, H,
+ * f1w [64][32], f1b, f2w [2][64], f2b; c2w, c3w and c4w 16-byte aligned.
+ * x: [B][H][W] BF16, 4-byte aligned, H % 16 == 0, W % 64 == 0; y: [B][2] FP32.  saved: device memory of lgm_cnn_net_bytes(B, H,
  * W, keep) bytes, 256-byte aligned; with keep != 0 it holds what the backward
  * call reads. */
 size_t lgm_cnn_net_bytes(int32_t B, int32_t H, int32_t W, int32_t which);

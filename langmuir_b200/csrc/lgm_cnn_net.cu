@@ -1057,8 +1057,9 @@ lgm_status lgm_cnn_net_forward(const void* x, const float* const* params, void* 
                                int32_t B, int32_t H, int32_t W, int32_t keep, void* stream) {
     if (!x || !params || !saved || !y || !shape_ok(B, H, W)) return LGM_ERR_INVALID_ARGUMENT;
     if (((uintptr_t)x & 3u) || ((uintptr_t)saved & 255u)) return LGM_ERR_INVALID_ARGUMENT;
-    for (int i = 0; i < 12; ++i)
-        if (!params[i]) return LGM_ERR_INVALID_ARGUMENT;
+    for (int i = 0; i < 12; ++i)  // conv_planes reads the masters of layers 2 to 4 as float4
+        if (!params[i] || ((uintptr_t)params[i] & (i == 2 || i == 4 || i == 6 ? 15u : 3u)))
+            return LGM_ERR_INVALID_ARGUMENT;
     Device d;
     lgm_status s = device_of(&d);
     if (s != LGM_OK) return s;
@@ -1093,7 +1094,8 @@ lgm_status lgm_cnn_net_backward(const void* x, const void* saved, const float* d
                                 int32_t W, void* stream) {
     if (!x || !saved || !dy || !work || !grads || !shape_ok(B, H, W))
         return LGM_ERR_INVALID_ARGUMENT;
-    if (((uintptr_t)saved & 255u) || ((uintptr_t)work & 255u)) return LGM_ERR_INVALID_ARGUMENT;
+    if (((uintptr_t)x & 3u) || ((uintptr_t)saved & 255u) || ((uintptr_t)work & 255u))
+        return LGM_ERR_INVALID_ARGUMENT;
     for (int i = 0; i < 12; ++i)
         if (!grads[i] || ((uintptr_t)grads[i] & 15u)) return LGM_ERR_INVALID_ARGUMENT;
     Device d;

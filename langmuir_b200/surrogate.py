@@ -186,10 +186,17 @@ def check_image_shape(H, W):
         raise ValueError(f"image {H}x{W}: the kernels need H % 64 == 0 and W % 128 == 0")
 
 
+def _aligned(t, nbytes):
+    """t as a contiguous tensor at a multiple of nbytes: itself, or a copy (a view into a
+    flat buffer may lie anywhere; fresh storage is aligned)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % nbytes == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 def _masters(params):
-    """The twelve FP32 masters as contiguous tensors and a C array of their pointers."""
-    ps = [p if p.dtype == torch.float32 and p.is_contiguous() else p.float().contiguous()
-          for p in params]
+    """The twelve FP32 masters as contiguous, 16-byte aligned tensors and a C array of their
+    pointers."""
+    ps = [_aligned(p.float(), 16) for p in params]
     return ps, (_vp * len(ps))(*[p.data_ptr() for p in ps])
 
 
@@ -198,7 +205,7 @@ def network_forward(x16, params, keep=True):
     Returns y [B,2] fp32 and (keep) what the backward pass reads."""
     B, H, W, _ = x16.shape
     check_image_shape(H, W)
-    x16 = x16.contiguous()
+    x16 = _aligned(x16, 4)
     masters, ptrs = _masters(params)
     work = torch.empty(N.lib().lgm_cnn_net_bytes(B, H, W, int(keep)), dtype=torch.uint8,
                        device=x16.device)
