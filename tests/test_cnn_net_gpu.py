@@ -73,3 +73,25 @@ def test_native_forward_has_the_layers_bits(n, H, W, seed):
                              relu=True))
         want = S.gemm(h, hid, 1, f2w.to(torch.bfloat16), 1, hid, n, out, hid, bias=f2b)
     np.testing.assert_array_equal(y.cpu().numpy(), want.cpu().numpy())
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+def test_non_finite_pixels_reach_their_neighbours_only(value):
+    """An infinity or NaN in an image does to its 3x3 neighbourhood what it does in
+    the per-layer kernels, and nothing to the pixels beside it."""
+    import torch
+    from langmuir_b200 import surrogate as S
+    H, W = 64, 128
+    at = [(0, 0), (5, 2), (5, 3), (10, 16), (10, 31), (11, 32), (20, 63), (33, 64), (63, 127),
+          (62, 126), (40, 127), (40, 1)]
+    x = S.phases_to_input(torch.zeros(len(at), H, W, dtype=torch.uint8), ramp=0.5)
+    for b, (r, c) in enumerate(at):
+        x[b, r, c] = value
+    params = [p.detach() for p in S.init_params(7)]
+    params[1].fill_(0.25)
+    y, (_, kept) = S.network_forward(x, params)
+    _, p1 = S.conv3x3(x, S.conv_weights_bf16(params[0], 1), params[1], H, W, keep_act=False)
+    # layer 1's pooled output, planes of eight channels, comes first in what is kept
+    planes = kept[:p1.numel() * 2].view(torch.bfloat16).view(len(at), 4, H // 2, W // 2, 8)
+    got = planes.permute(0, 2, 3, 1, 4).reshape(p1.shape)
+    np.testing.assert_array_equal(got.float().cpu().numpy(), p1.float().cpu().numpy())
