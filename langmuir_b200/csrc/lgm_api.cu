@@ -871,16 +871,18 @@ SmallFn small_fn(int kind, int path) {
 }
 
 // A call of few sources takes the one-kernel form (lgm_small.cuh): up to
-// kSmallSources of them and kSmallPairs unculled pairs, where the chain's
+// kSmallSources of them and small_pairs unculled pairs, where the chain's
 // launches cost more than the pairs it culls, with no variant forced or tuned
 // for the size (the FP64 precision has none), no pair counting, and a table
 // that leaves two CTAs their shared memory.
-bool small_call(const lgm_ctx* c, int kind, const Shape& sh, int n, int t) {
-    const bool f64 = c->cfg.precision == LGM_PREC_FP64;
+bool small_call(const lgm_ctx* c, int kind, const Shape& sh, int n, int t, bool all_sites) {
+    const bool f64 = c->cfg.precision == LGM_PREC_FP64, fp64_terms = sum_path(c) == LGM_PATH_TABLE64;
     if (f64 ? !f64_table(c) : c->forced_variant >= 0 || c->counting) return false;
-    if (n < 1 || n > kSmallSources || (long long)n * t * sh.nterms > kSmallPairs) return false;
+    if (n < 1 || n > kSmallSources ||
+        (long long)n * t * sh.nterms > small_pairs(n, fp64_terms, all_sites))
+        return false;
     if (!f64 && c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks))) return false;
-    return small_smem(n, small_table(c, kind), sum_path(c) == LGM_PATH_TABLE64 ? 8 : 4) <= kSmallSmem;
+    return small_smem(n, small_table(c, kind), fp64_terms ? 8 : 4) <= kSmallSmem;
 }
 
 // flag: null, or the host-visible word the last CTA writes {call, error} to.
@@ -957,7 +959,7 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     }
     const Shape sh = shape_of(n, t, terms);
     // (err_out: the host-buffer call, which takes the small form itself)
-    if (!err_out && small_call(c, kind, sh, n, t))
+    if (!err_out && small_call(c, kind, sh, n, t, all_sites))
         return launch_small(c, kind, terms, d_src, d_q, n, d_tgt_site, t, all_sites, d_out, st, nullptr,
                             0);
     const bool f64 = cf.precision == LGM_PREC_FP64, direct = f64 && !f64_table(c);
@@ -1524,7 +1526,7 @@ lgm_status lgm_potentials(lgm_ctx* c, lgm_kind kind, uint32_t terms, const int32
     if ((s = grow_device(c, &c->d_t, &c->t_cap, words)) != LGM_OK) return s;
     if ((s = grow_device(c, &c->d_o, &c->o_cap, (size_t)t + 1)) != LGM_OK) return s;
     const Shape sh = shape_of(n, t, terms);
-    const bool small = n > 0 && small_call(c, kind, sh, n, t);
+    const bool small = n > 0 && small_call(c, kind, sh, n, t, false);
     // The sites are checked on the device (prep_records), which gives each an
     // empty record and raises an error bit; only then are they checked here,
     // for the first bad one (sources first, then targets, as check_sites

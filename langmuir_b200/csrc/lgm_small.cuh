@@ -21,8 +21,22 @@ namespace lgm {
 
 constexpr int kSmallThreads = 256, kSmallWarps = kSmallThreads / 32;
 constexpr size_t kSmallSmem = 96 * 1024;  // dynamic shared memory, at most
-constexpr int kSmallSources = 2048;       // a sort of 2048 keys takes a CTA about 4 us
-constexpr long long kSmallPairs = 1 << 25;  // unculled pairs of a call: about 13 us of the GPU
+// Sources and unculled pairs of a call in this form, at most (small_pairs); its sort's
+// places in s_list and the index in its keys hold 2048.
+constexpr int kSmallSources = 2048;
+inline long long small_pairs(int n, bool fp64, bool all_sites) {
+    // The chain sorts the targets too, and culls; this form sorts the sources again in
+    // every CTA, by counting up to 512 of them, in some microseconds more beyond that.
+    // us a device call, this form and the chain, 256x256x16, cutoff 50:
+    //   128 sources, 2^27 pairs 63 and 298; 512, 2^26 58 and 56, 2^27 72 and 85
+    //   1024 sources, 2^24 pairs 28 and 31, 2^25 33 and 34, 2^27 77 and 61
+    //   1500 sources, 2^22 pairs 31 and 30, 2^23 43 and 30; 2048, 2^22 34 and 30 (host
+    //   call 55 and 54), 2^25 52 and 33
+    // Every site: a segment is a run along x and culls well; 1000 sources on 2^20 sites
+    // 139 and 204.  Terms from FP64 tables: 400 sources, 2^25 pairs 57 and 55.
+    if (!fp64 && n <= (all_sites ? 1024 : 512)) return 1ll << 62;
+    return n <= 1024 ? 1ll << 25 : 1ll << 22;
+}
 
 struct SmallArgs {
     const int32_t *src, *q;   // n sources
