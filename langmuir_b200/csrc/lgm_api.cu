@@ -628,30 +628,119 @@ Shape shape_of(int n, int t, unsigned terms) {
     return sh;
 }
 
+// Slices one after another of a block, 256-byte aligned; without a block, their bytes.
+struct Cut {
+    char* base;
+    size_t at;
+    template <class T>
+    void operator()(T** p, size_t n) {
+        if (base) *p = reinterpret_cast<T*>(base + at);
+        at += (n * sizeof(T) + 255) / 256 * 256;
+    }
+};
+
+// The sort of n sources and t targets, and their records.
+void cut_records(lgm_ctx* c, Cut& cut, const Shape& sh, int n, int t, int fmt) {
+    const size_t ns = (size_t)sh.n_pad + kGroup;
+    if (fmt & kFmtFloat) {
+        cut(&c->d_geo, (size_t)sh.n_pad * 2);
+        cut(&c->d_qq, (size_t)sh.n_pad);
+        cut(&c->d_tgt, (size_t)sh.t_phys + 4096);  // room for any variant's widest tile
+    }
+    if (fmt & kFmtHalf) {
+        cut(&c->d_frag, ns * 4);
+        cut(&c->d_q1, ns);
+        cut(&c->d_tgt16, (size_t)sh.t_phys);  // whole segments: t_pad is a multiple of 64
+    }
+    cut(&c->d_key, (size_t)t);
+    cut(&c->d_perm, (size_t)t);
+    cut(&c->d_ttmp, (size_t)t);
+    cut(&c->d_skey, (size_t)n);
+    cut(&c->d_stmp, (size_t)n);
+}
+
+// Sizes of a culled variant's work lists.
+struct CulledPlan {
+    int tile, tiles, per_item, max_items, mask_stride;
+    size_t item_cap;
+};
+CulledPlan culled_plan(const Variant& V, const Shape& sh) {
+    CulledPlan p;
+    p.tile = variant_tile(V);
+    p.tiles = (sh.t_phys + p.tile - 1) / p.tile;
+    p.per_item = V.per_item;
+    if (V.tc)
+        mma_items(p.tiles, sh.n_chunks * kGroupsPerChunk, false, &p.per_item, &p.max_items);
+    else
+        p.max_items =
+            std::max(1, std::min(kMaxItemsPerTile, (sh.n_chunks + p.per_item - 1) / p.per_item));
+    p.mask_stride = (sh.n_chunks + 31) / 32 * 32;
+    p.item_cap = (size_t)p.tiles * p.max_items;
+    return p;
+}
+
+int splits_for(const lgm_ctx* c, int v, int fi, const Shape& sh, int* tiles_out);
+int direct_splits(const lgm_ctx* c, const Shape& sh);
+constexpr int kDirect = -1;  // in place of a variant: pair_kernel_f64
+
+// The pair sum of variant v (or kDirect): boxes, live lists, items, partial sums.
+void cut_sums(lgm_ctx* c, Cut& cut, const Shape& sh, int v, int fi) {
+    if (v == kDirect || !kVariants[v].cull) {
+        int tiles;
+        const int splits = v == kDirect ? direct_splits(c, sh) : splits_for(c, v, fi, sh, &tiles);
+        cut(&c->d_part, (size_t)splits * sh.t_phys);
+        return;
+    }
+    const Variant& V = kVariants[v];
+    const CulledPlan p = culled_plan(V, sh);
+    cut(&c->d_cbox, (size_t)sh.n_chunks);
+    cut(&c->d_gbox, (size_t)sh.n_chunks * kGroupsPerChunk);
+    if (V.tc) {
+        cut(&c->d_gmask, (size_t)p.tiles * p.mask_stride);
+    } else {
+        cut(&c->d_live, (size_t)p.tiles * sh.n_chunks);
+        cut(&c->d_order, p.item_cap);
+        cut(&c->d_oitems, p.item_cap);
+    }
+    cut(&c->d_items, p.item_cap);
+    cut(&c->d_tile_first, (size_t)p.tiles);
+    cut(&c->d_tile_items, (size_t)p.tiles);
+    cut(&c->d_part, p.item_cap * p.tile);
+}
+
+// The scratch of a call, records in format fmt and any of the variants vs; the
+// slices of the sums are cut again for each variant.  A new context's first call
+// pays for the allocations: the driver serves up to 1 MB in 2 us from pieces of
+// 2 MB that it holds, and maps anything larger in 330.  So a call of at most 2 MB
+// takes two blocks, a larger one takes one.
+constexpr size_t kTwoBlocks = 2 << 20;
+lgm_status lay_out(lgm_ctx* c, const Shape& sh, int n, int t, int fmt, int fi,
+                   const std::vector<int>& vs) {
+    Cut dry{nullptr, 0};
+    cut_records(c, dry, sh, n, t, fmt);
+    const size_t records = dry.at;
+    size_t need = records;
+    for (int v : vs) {
+        dry.at = records;
+        cut_sums(c, dry, sh, v, fi);
+        need = std::max(need, dry.at);
+    }
+    const bool one = need <= c->scratch_cap || need > kTwoBlocks;
+    lgm_status s = grow_device(c, &c->d_scratch, &c->scratch_cap, one ? need : records);
+    if (s == LGM_OK && !one) s = grow_device(c, &c->d_sums, &c->sums_cap, need - records);
+    if (s != LGM_OK) return s;
+    c->sums = one ? c->d_scratch + records : c->d_sums;
+    Cut cut{c->d_scratch, 0};
+    cut_records(c, cut, sh, n, t, fmt);
+    return LGM_OK;
+}
+
+// Sorts and writes the records of a call that lay_out made room for.
 lgm_status prep(lgm_ctx* c, unsigned terms, const int32_t* d_src, const int32_t* d_q, int n,
                 const int32_t* d_tgt_site, int t, int all_sites, const Shape& sh, int fmt,
                 cudaStream_t st) {
     const lgm_config& cf = c->cfg;
-    lgm_status s;
-    // target records: room for the widest target tile of any variant
-    const size_t tgt_n = (size_t)sh.t_phys + 4096;
-    if (fmt & kFmtFloat) {
-        if ((s = grow_device(c, &c->d_geo, &c->geo_cap, (size_t)sh.n_pad * 2)) != LGM_OK) return s;
-        if ((s = grow_device(c, &c->d_qq, &c->qq_cap, (size_t)sh.n_pad)) != LGM_OK) return s;
-        if ((s = grow_device(c, &c->d_tgt, &c->tgt_cap, tgt_n)) != LGM_OK) return s;
-    }
-    if (fmt & kFmtHalf) {
-        const size_t ns = (size_t)sh.n_pad + kGroup;
-        if ((s = grow_device(c, &c->d_frag, &c->frag_cap, ns * 4)) != LGM_OK) return s;
-        if ((s = grow_device(c, &c->d_q1, &c->q1_cap, ns)) != LGM_OK) return s;
-        if ((s = grow_device(c, &c->d_tgt16, &c->tgt16_cap, tgt_n)) != LGM_OK) return s;
-    }
     const Records R{fmt, c->d_geo, c->d_qq, c->d_tgt, c->d_frag, c->d_q1, c->d_tgt16};
-    if ((s = grow_device(c, &c->d_key, &c->key_cap, (size_t)t)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_perm, &c->perm_cap, (size_t)t)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_ttmp, &c->ttmp_cap, (size_t)t)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_skey, &c->skey_cap, (size_t)n)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_stmp, &c->stmp_cap, (size_t)n)) != LGM_OK) return s;
     // targets and sources in spatial order: bins, scans, scatters.  Both bin
     // arrays and the bins_both block counter behind them start at zero: the
     // last kernel of the previous call cleared them (bins_both's last block
@@ -692,37 +781,24 @@ int splits_for(const lgm_ctx* c, int v, int fi, const Shape& sh, int* tiles_out)
     return std::max(1, std::min({kMaxSplits, kSplitWaves * capacity / tiles, sh.n_chunks}));
 }
 
+// Splits of the source range for pair_kernel_f64.
+int direct_splits(const lgm_ctx* c, const Shape& sh) {
+    const int ctas = (sh.t_phys + kF64Threads - 1) / kF64Threads;
+    return std::max(1, std::min({kMaxSplits, (c->sm_count * 8) / std::max(1, ctas),
+                                 (sh.n_pad + kF64Tile - 1) / kF64Tile}));
+}
+
 // Culled variant v: chunk boxes, the cull, the persistent pair kernel (one
 // wave of resident CTAs).  *splits_out = 0 tells the caller to finalize from
 // the item partials.
 lgm_status launch_culled(lgm_ctx* c, int fi, int v, const Shape& sh, const PairArgs& A,
                          cudaStream_t st, int* splits_out) {
     const Variant& V = kVariants[v];
-    const int TS = variant_tile(V);
-    const int tiles = (sh.t_phys + TS - 1) / TS;
-    const int grid = c->sm_count * std::max(1, c->bps[v][fi]);
-    int per_item = V.per_item, max_items = kMaxItemsPerTile;
-    if (V.tc) mma_items(tiles, sh.n_chunks * kGroupsPerChunk, false, &per_item, &max_items);
-    else max_items = std::max(1, std::min(max_items, (sh.n_chunks + per_item - 1) / per_item));
-    const int mask_stride = (sh.n_chunks + 31) / 32 * 32;
+    const CulledPlan p = culled_plan(V, sh);
+    const int tiles = p.tiles, grid = c->sm_count * std::max(1, c->bps[v][fi]);
     if (V.nt / 32 > kMaxSegments) return fail(c, LGM_ERR_STATE, "culled variant wider than the cull");
-    const size_t item_cap = (size_t)tiles * max_items;
-    lgm_status s;
-    if ((s = grow_device(c, &c->d_cbox, &c->cbox_cap, (size_t)sh.n_chunks)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_gbox, &c->gbox_cap, (size_t)sh.n_chunks * kGroupsPerChunk)) !=
-        LGM_OK)
-        return s;
-    if (V.tc) s = grow_device(c, &c->d_gmask, &c->gmask_cap, (size_t)tiles * mask_stride);
-    else s = grow_device(c, &c->d_live, &c->live_cap, (size_t)tiles * sh.n_chunks);
-    if (s != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_items, &c->items_cap, item_cap)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_tile_first, &c->tfirst_cap, (size_t)tiles)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_tile_items, &c->titems_cap, (size_t)tiles)) != LGM_OK) return s;
-    if ((s = grow_device(c, &c->d_part, &c->part_cap, item_cap * TS)) != LGM_OK) return s;
-    if (!V.tc) {
-        if ((s = grow_device(c, &c->d_order, &c->order_cap, item_cap)) != LGM_OK) return s;
-        if ((s = grow_device(c, &c->d_oitems, &c->oitems_cap, item_cap)) != LGM_OK) return s;
-    }
+    Cut cut{c->sums, 0};
+    cut_sums(c, cut, sh, v, fi);
     PairArgs P = A;
     P.part = c->d_part;
     CullArgs C;
@@ -732,13 +808,13 @@ lgm_status launch_culled(lgm_ctx* c, int fi, int v, const Shape& sh, const PairA
     C.tgt = c->d_tgt;
     C.t_phys = sh.t_phys;
     C.c2 = c->cfg.electrostatic_cutoff * c->cfg.electrostatic_cutoff;
-    C.tile_size = TS;
-    C.per_item = per_item;
-    C.max_items = max_items;
+    C.tile_size = p.tile;
+    C.per_item = p.per_item;
+    C.max_items = p.max_items;
     C.live = c->d_live;
     C.tgt16 = c->d_tgt16;
     C.gmask = c->d_gmask;
-    C.mask_stride = mask_stride;
+    C.mask_stride = p.mask_stride;
     C.max_tiles = tiles;
     C.live_stride = sh.n_chunks;
     C.items = c->d_items;
@@ -806,9 +882,8 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int path, int v, const Shape& sh, c
     }
     int tiles;
     const int splits = splits_for(c, v, fi, sh, &tiles);
-    lgm_status s;
-    if ((s = grow_device(c, &c->d_part, &c->part_cap, (size_t)splits * sh.t_phys)) != LGM_OK)
-        return s;
+    Cut cut{c->sums, 0};
+    cut_sums(c, cut, sh, v, fi);
     PairArgs A;
     A.geo = c->d_geo; A.qq = c->d_qq; A.n_chunks = sh.n_chunks; A.splits = splits;
     A.tgt = c->d_tgt; A.t_phys = sh.t_phys; A.part = c->d_part;
@@ -966,6 +1041,8 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     const int v = f64 ? kDefaultVariant : choose_variant(c, kind, sh);
     const int fmt = direct || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
     lgm_status s;
+    if ((s = lay_out(c, sh, n, t, fmt, fn_index(kind, sum_path(c)), {direct ? kDirect : v})) != LGM_OK)
+        return s;
     if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, fmt, st)) != LGM_OK)
         return s;
     int splits = 1;
@@ -973,12 +1050,10 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     if (direct) {
         const double erffactor =
             cf.coulomb_gaussian_sigma > 0 ? 1.0 / (std::sqrt(2.0) * cf.coulomb_gaussian_sigma) : 0.0;
-        const int ctas = (sh.t_phys + kF64Threads - 1) / kF64Threads;
-        splits = std::max(1, std::min({kMaxSplits, (c->sm_count * 8) / std::max(1, ctas),
-                                       (sh.n_pad + kF64Tile - 1) / kF64Tile}));
-        if ((s = grow_device(c, &c->d_part, &c->part_cap, (size_t)splits * sh.t_phys)) != LGM_OK)
-            return s;
-        dim3 grid(ctas, splits);
+        splits = direct_splits(c, sh);
+        Cut cut{c->sums, 0};
+        cut_sums(c, cut, sh, kDirect, 0);
+        dim3 grid((sh.t_phys + kF64Threads - 1) / kF64Threads, splits);
         LGM_CUDA(c, launch_chain(c->overlap, pair_kernel_f64, grid, kF64Threads, 0, st, c->d_geo,
                                  c->d_qq, sh.n_pad, splits, c->d_tgt, sh.t_phys, c->d_part,
                                  cf.electrostatic_cutoff * cf.electrostatic_cutoff, kind,
@@ -1327,15 +1402,9 @@ lgm_status lgm_destroy(lgm_ctx* c) {
     if (!c) return LGM_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void* dev_ptrs[] = {c->d_geo,   c->d_qq,         c->d_tgt,        c->d_part,
-                        c->d_s,     c->d_q,          c->d_t,          c->d_o,
-                        c->d_gtab,  c->d_rtab,       c->d_err,        c->d_cell_rank,
-                        c->d_bins,  c->d_key,        c->d_perm,       c->d_ttmp,
-                        c->d_skey,  c->d_stmp,       c->d_cbox,       c->d_gbox,
-                        c->d_live,  c->d_items,      c->d_tile_first, c->d_tile_items,
-                        c->d_item_count, c->d_examined, c->d_rtab64,  c->d_gtab64,
-                        c->d_cost_hist,  c->d_order,     c->d_oitems,     c->d_frag,
-                        c->d_q1,         c->d_tgt16,     c->d_gmask};
+    void* dev_ptrs[] = {c->d_scratch, c->d_sums, c->d_s,        c->d_q,      c->d_t,         c->d_o,
+                        c->d_gtab,    c->d_rtab,     c->d_rtab64, c->d_gtab64,    c->d_err,
+                        c->d_cell_rank, c->d_bins,   c->d_item_count, c->d_examined, c->d_cost_hist};
     for (void* p : dev_ptrs)
         if (p) cudaFree(p);
     void* host_ptrs[] = {c->h_s, c->h_q, c->h_t, c->h_o, c->h_err};
@@ -1452,16 +1521,19 @@ lgm_status lgm_autotune(lgm_ctx* c, lgm_kind kind, uint32_t terms, int32_t n, in
     LGM_CUDA(c, cudaMemcpyAsync(c->d_q, hq.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
     LGM_CUDA(c, cudaMemcpyAsync(c->d_t, ht.data(), sizeof(int32_t) * t, cudaMemcpyHostToDevice, st));
     const Shape sh = shape_of(n, t, terms);
-    if ((s = prep(c, terms, c->d_s, c->d_q, n, c->d_t, t, 0, sh, kFmtFloat | kFmtHalf, st)) !=
-        LGM_OK)
+    std::vector<int> vs;
+    for (int v = 0; v < kNumVariants; ++v)
+        if (c->cfg.path != LGM_PATH_TABLE64 || kVariants[v].cull) vs.push_back(v);
+    if ((s = lay_out(c, sh, n, t, kFmtFloat | kFmtHalf, fn_index(kind, c->cfg.path), vs)) != LGM_OK ||
+        (s = prep(c, terms, c->d_s, c->d_q, n, c->d_t, t, 0, sh, kFmtFloat | kFmtHalf, st)) !=
+            LGM_OK)
         return s;
     cudaEvent_t e0, e1;
     LGM_CUDA(c, cudaEventCreate(&e0));
     LGM_CUDA(c, cudaEventCreate(&e1));
     int best = kDefaultVariant;
     float best_ms = 1e30f;
-    for (int v = 0; v < kNumVariants; ++v) {
-        if (c->cfg.path == LGM_PATH_TABLE64 && !kVariants[v].cull) continue;
+    for (int v : vs) {
         int splits;
         if ((s = launch_pair(c, kind, c->cfg.path, v, sh, st, &splits)) != LGM_OK) break;  // warm
         float ms[3];

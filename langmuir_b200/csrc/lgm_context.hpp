@@ -17,16 +17,21 @@ struct lgm_ctx {
     int xy = 0;
     cudaStream_t stream = nullptr;
 
-    // Device work buffers, grown on demand (never inside stream capture).
-    float4* d_geo = nullptr;  size_t geo_cap = 0;   // 2 float4 per source
-    float2* d_qq = nullptr;   size_t qq_cap = 0;    // 1 float2 per source
-    float4* d_tgt = nullptr;  size_t tgt_cap = 0;   // per physical target
+    // Scratch of a chain of kernels: one or two blocks, cut into the slices that the
+    // call's size and variant need (lay_out, lgm_api.cu).  Nothing in them outlives a
+    // call.  They grow on demand (never inside stream capture).
+    char* d_scratch = nullptr; size_t scratch_cap = 0;
+    char* d_sums = nullptr;    size_t sums_cap = 0;
+    char* sums = nullptr;               // where the slices of the pair sum begin
+    float4* d_geo = nullptr;            // 2 float4 per source
+    float2* d_qq = nullptr;             // 1 float2 per source
+    float4* d_tgt = nullptr;            // per physical target
     // tensor-core sums (lgm_mma.cuh): source fragments, charges, target rows, live groups
-    uint32_t* d_frag = nullptr; size_t frag_cap = 0;
-    float* d_q1 = nullptr;    size_t q1_cap = 0;
-    uint4* d_tgt16 = nullptr; size_t tgt16_cap = 0;
-    uint8_t* d_gmask = nullptr; size_t gmask_cap = 0;
-    double* d_part = nullptr; size_t part_cap = 0;  // split partial sums
+    uint32_t* d_frag = nullptr;
+    float* d_q1 = nullptr;
+    uint4* d_tgt16 = nullptr;
+    uint8_t* d_gmask = nullptr;
+    double* d_part = nullptr;           // split or item partial sums
     int32_t* d_s = nullptr;   size_t s_cap = 0;     // staging for host-buffer calls
     int32_t* d_q = nullptr;   size_t q_cap = 0;
     int32_t* d_t = nullptr;   size_t t_cap = 0;
@@ -43,32 +48,32 @@ struct lgm_ctx {
     int cell_shift = 2, cells_x = 0, cells_y = 0, ncells = 0;
     int32_t* d_cell_rank = nullptr;                  // [ncells]
     int32_t* d_bins = nullptr;                       // [ncells + 2] counts, then offsets
-    int32_t* d_key = nullptr;  size_t key_cap = 0;   // bin per target
-    int32_t* d_perm = nullptr; size_t perm_cap = 0;  // target of each physical slot
-    int32_t* d_ttmp = nullptr; size_t ttmp_cap = 0;  // targets scattered by bin
+    int32_t* d_key = nullptr;   // bin per target
+    int32_t* d_perm = nullptr;  // target of each physical slot
+    int32_t* d_ttmp = nullptr;  // targets scattered by bin
     // The sources in the same spatial order: bin per source (d_sbins follows
     // the target bins in the d_bins allocation), the sources scattered by bin,
     // then ranked inside their bin by (site, index), so that the order is a
     // function of the sources alone.
     int32_t* d_sbins = nullptr;                       // [ncells + 2], inside d_bins
     int bins_stride = 0;                              // ncells + 2 rounded up to 4
-    int32_t* d_skey = nullptr; size_t skey_cap = 0;   // bin per source
-    int32_t* d_stmp = nullptr; size_t stmp_cap = 0;   // sources scattered by bin
+    int32_t* d_skey = nullptr;   // bin per source
+    int32_t* d_stmp = nullptr;   // sources scattered by bin
     // Culled pair sums (lgm_cull.cuh): chunk and group boxes, live chunk
     // lists per tile, work items, and where each tile's items start.
-    int4* d_cbox = nullptr;  size_t cbox_cap = 0;     // lgm::Box per chunk
-    int4* d_gbox = nullptr;  size_t gbox_cap = 0;     // lgm::Box per 32-source group
-    int32_t* d_live = nullptr; size_t live_cap = 0;
-    int4* d_items = nullptr; size_t items_cap = 0;
-    int32_t* d_tile_first = nullptr; size_t tfirst_cap = 0;
-    int32_t* d_tile_items = nullptr; size_t titems_cap = 0;
+    int4* d_cbox = nullptr;     // lgm::Box per chunk
+    int4* d_gbox = nullptr;     // lgm::Box per 32-source group
+    int32_t* d_live = nullptr;
+    int4* d_items = nullptr;
+    int32_t* d_tile_first = nullptr;
+    int32_t* d_tile_items = nullptr;
     int32_t* d_item_count = nullptr;                  // [4]: items written, next item taken,
                                                       // tiles culled; CTAs of a one-kernel
                                                       // call done
     unsigned call_number = 0;                         // one-kernel host-buffer calls made
     int32_t* d_cost_hist = nullptr;                   // [kCostBuckets] items per cost
-    int32_t* d_order = nullptr; size_t order_cap = 0; // items by decreasing cost
-    int4* d_oitems = nullptr; size_t oitems_cap = 0;  // their records in that order
+    int32_t* d_order = nullptr; // items by decreasing cost
+    int4* d_oitems = nullptr;  // their records in that order
 
     // Pinned host staging for the host-buffer entry points.
     int32_t* h_s = nullptr;   size_t hs_cap = 0;
