@@ -662,7 +662,7 @@ void cut_records(lgm_ctx* c, Cut& cut, const Shape& sh, int n, int t, int fmt) {
 // Sizes of a culled variant's work lists.
 struct CulledPlan {
     int tile, tiles, per_item, max_items, mask_stride;
-    size_t item_cap;
+    size_t item_cap;  // room for items: never less than a smaller call's
 };
 CulledPlan culled_plan(const Variant& V, const Shape& sh) {
     CulledPlan p;
@@ -675,7 +675,8 @@ CulledPlan culled_plan(const Variant& V, const Shape& sh) {
         p.max_items =
             std::max(1, std::min(kMaxItemsPerTile, (sh.n_chunks + p.per_item - 1) / p.per_item));
     p.mask_stride = (sh.n_chunks + 31) / 32 * 32;
-    p.item_cap = (size_t)p.tiles * p.max_items;
+    p.item_cap = V.tc ? mma_item_room(p.tiles, sh.n_chunks * kGroupsPerChunk)
+                      : (size_t)p.tiles * p.max_items;
     return p;
 }
 

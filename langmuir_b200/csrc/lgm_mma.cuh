@@ -444,6 +444,16 @@ inline void mma_items(long long segs, int groups, bool batch, int* per_item, int
     *max_items = std::min(groups / per + 1, segs > 8192 ? kMaxItemsPerSeg / 2 : kMaxItemsPerSeg);
 }
 
+// Items that a call of at most so many segments and groups writes, at most (not in
+// a batch).  Fewer segments may mean more items: room by this bound serves every
+// smaller call too, such as one captured after a larger one has run.
+inline size_t mma_item_room(long long segs, int groups) {
+    const long long most = groups / kGroupsPerChunk + 1;  // items are never smaller
+    const long long few = std::min<long long>(segs, 8192) * std::min<long long>(kMaxItemsPerSeg, most);
+    const long long many = segs > 8192 ? segs * std::min<long long>(kMaxItemsPerSeg / 2, most) : 0;
+    return (size_t)std::max(few, many);
+}
+
 template <int KIND, int PATH, int LM, bool NORM = false>
 __global__ void __launch_bounds__(kMmaThreads, PATH == 2 ? kMmaCtas - 1 : kMmaCtas) pair_kernel_mma(PairArgs A, CullArgs C) {
     pdl_wait();

@@ -53,3 +53,38 @@ def test_variants_and_tuning_share_a_context(lgm):
         tuned = ctx.potentials(src, q, tgt, terms=7)
         ctx.set_counting(True)
         np.testing.assert_array_equal(ctx.potentials(src, q, tgt, terms=7), tuned)
+
+
+@pytest.mark.parametrize("n,warm,sizes", [(10000, 300000, (262000, 70000, 9000)),
+                                          (4000, 262400, (262100, 131000)),
+                                          (2622, 5244, (5000, 700))])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_smaller_calls_are_captured_after_a_larger_one(lgm, n, warm, sizes, precision):
+    """A captured call allocates nothing when a larger one has run, though fewer targets
+    may be cut into more items (8192 segments of 32 targets are a line of that)."""
+    import torch
+    X, Y, Z = 128, 128, 24
+    rng = np.random.default_rng(n)
+    host = (rng.choice(X * Y * Z, n, replace=False).astype(np.int32),
+            rng.choice([-1, 1], n).astype(np.int32),
+            rng.integers(0, X * Y * Z, warm).astype(np.int32))
+    src, q, tgt = (torch.as_tensor(a).cuda() for a in host)
+    out = torch.zeros(warm, dtype=torch.float64, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with lgm.Coulomb(X, Y, Z, cutoff=20, precision=precision) as ctx:
+        def call(t):
+            ctx.potentials_async(src.data_ptr(), q.data_ptr(), n, tgt.data_ptr(), t,
+                                 out.data_ptr(), stream=stream.cuda_stream)
+        call(warm)
+        ctx.sync(stream.cuda_stream)
+        for t in sizes:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=stream):
+                call(t)
+            out.zero_()
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            got = out[:t].cpu().numpy()
+            np.testing.assert_array_equal(got, ctx.potentials(*host[:2], host[2][:t]))
