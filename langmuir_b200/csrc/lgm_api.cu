@@ -566,11 +566,11 @@ const Variant kVariants[] = {
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 static_assert(kNumVariants <= (int)(sizeof(lgm_ctx::bps) / sizeof(lgm_ctx::bps[0])),
               "lgm_ctx::bps holds every variant");
-// warp-specialised culled, 4 target warps, 2 target pairs, runs of 16, 2
-// chunks per item, one vote per 2 sources (2% faster than a vote per source
-// on the 256x256x16 and 128x128x64 workloads, the same bits)
-// r^2 on the tensor cores
-constexpr int kDefaultVariant = kNumVariants - 1;
+// The defaults (choose_variant): r^2 on the tensor cores; for large calls with
+// tables the warp-specialised culled tile with 4 target warps, 2 target pairs, runs
+// of 16, 2 chunks per item and one vote per 2 sources (2% faster than a vote per
+// source on the 256x256x16 and 128x128x64 workloads, the same bits).
+constexpr int kDefaultVariant = kNumVariants - 1, kTileVariant = 32;
 
 // The culled kernel of variant V for path index fi and cutoff^2 c2.
 CulledFn culled_fn(const Variant& V, int fi, int c2) {
@@ -908,8 +908,36 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int path, int v, const Shape& sh, c
     return LGM_OK;
 }
 
-int choose_variant(const lgm_ctx* c, int kind, const Shape& sh) {
-    int v = kDefaultVariant;
+// Untuned calls with terms from tables that the FP32 tile (kTileVariant) sums
+// faster than the tensor-core kernel: its vote skips a table read that no lane of
+// the warp needs, where the other's conflicting reads bound it.  `inside` is about
+// the pairs within the cutoff.  us a device call, tile and tensor-core kernel:
+//   table64, cutoff 50: 2000 sources, 16,000 targets of 256x256x16 54 and 43; 6000,
+//   12,000 of 64x64x64 (inside 2^26) 103 and 104; 20,000, 40,000 (2^29) 605 and 667;
+//   every site of 64x64x64, 2000 sources 460 and 504, of 256x256x16, 600: 217 and 264
+//   table64, cutoff 100: 2000 and 4000 of 128x128x32 (2^22) 56 and 45; 2000 and
+//   16,000 (2^24) 70 and 76
+//   table, cutoff 150: 2000 and 4000 of 128x128x32 1.14 to 1.18 times faster by the
+//   latter; 2000 and 16,000 (2^24) 59 and 64; every site of 64x64x64, cutoff 50,
+//   2000 sources 323 and 335
+// With terms from the MUFU the tensor-core kernel is never more than 4% behind; but
+// its masks grow as targets x sources, twice as fast as the tile's lists, and are
+// left alone past 64 GB.
+bool tile_faster(const lgm_ctx* c, const Shape& sh, int n) {
+    const lgm_config& cf = c->cfg;
+    if ((long long)(sh.t_phys / kSeg) * sh.n_chunks > 1ll << 36) return true;
+    if (cf.path == LGM_PATH_RSQRT) return false;
+    double inside = (double)sh.t_phys * n;
+    for (int side : {cf.grid_x, cf.grid_y, cf.grid_z})
+        inside *= std::min(1.0, 2.0 * cf.electrostatic_cutoff / side);
+    if (cf.path == LGM_PATH_TABLE64)
+        return sh.t_phys > 65536 || inside > (cf.electrostatic_cutoff > 60 ? 0x1p24 : 0x1p27);
+    return (cf.electrostatic_cutoff >= 40 && sh.t_phys > 200000) ||
+           (cf.electrostatic_cutoff > 110 && inside > 0x1p24);
+}
+
+int choose_variant(const lgm_ctx* c, int kind, const Shape& sh, int n) {
+    int v = tile_faster(c, sh, n) ? kTileVariant : kDefaultVariant;
     if (c->forced_variant >= 0) {
         v = c->forced_variant;
     } else {
@@ -1039,10 +1067,16 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
         return launch_small(c, kind, terms, d_src, d_q, n, d_tgt_site, t, all_sites, d_out, st, nullptr,
                             0);
     const bool f64 = cf.precision == LGM_PREC_FP64, direct = f64 && !f64_table(c);
-    const int v = f64 ? kDefaultVariant : choose_variant(c, kind, sh);
+    const int v = f64 ? kDefaultVariant : choose_variant(c, kind, sh, n);
     const int fmt = direct || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
     lgm_status s;
-    if ((s = lay_out(c, sh, n, t, fmt, fn_index(kind, sum_path(c)), {direct ? kDirect : v})) != LGM_OK)
+    // an untuned call with tables makes room for both default variants: a smaller
+    // one may take the other
+    const bool both = !f64 && cf.path != LGM_PATH_RSQRT && c->forced_variant < 0;
+    std::vector<int> vs = {direct ? kDirect : v};
+    if (both) vs = {v, kDefaultVariant, kTileVariant};
+    if ((s = lay_out(c, sh, n, t, both ? kFmtFloat | kFmtHalf : fmt, fn_index(kind, sum_path(c)), vs)) !=
+        LGM_OK)
         return s;
     if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, fmt, st)) != LGM_OK)
         return s;

@@ -88,3 +88,43 @@ def test_smaller_calls_are_captured_after_a_larger_one(lgm, n, warm, sizes, prec
             torch.cuda.synchronize()
             got = out[:t].cpu().numpy()
             np.testing.assert_array_equal(got, ctx.potentials(*host[:2], host[2][:t]))
+
+
+@pytest.mark.parametrize("dims,cutoff,path,n,t,tile", [
+    ((64, 64, 32), 50, 2, 2100, 32000, False), ((64, 64, 32), 50, 2, 2100, 65536, True),
+    ((64, 64, 32), 50, 2, 2100, 66000, True), ((128, 128, 16), 20, 2, 2100, 65000, False),
+    ((128, 128, 16), 20, 2, 2100, 66000, True), ((64, 64, 32), 100, 2, 2100, 7900, False),
+    ((64, 64, 32), 100, 2, 2100, 8100, True), ((64, 64, 32), 100, 1, 2100, 8100, False),
+    ((64, 64, 32), 150, 1, 2100, 7900, False), ((64, 64, 32), 150, 1, 2100, 8100, True),
+    ((64, 64, 32), 40, 1, 2100, 199900, False), ((64, 64, 32), 40, 1, 2100, 200100, True),
+    ((64, 64, 32), 39, 1, 2100, 200100, False), ((64, 64, 32), 150, 0, 2100, 250000, False)])
+def test_which_kernel_sums_from_tables(lgm, dims, cutoff, path, n, t, tile):
+    """Both sides of the lines between the two default kernels, which add the same FP32
+    runs (or FP64 terms) in another order of FP64 sums; a smaller call on the same
+    context may take the other kernel, under capture too."""
+    import torch
+    rng = np.random.default_rng(t)
+    sites = dims[0] * dims[1] * dims[2]
+    src = rng.choice(sites, n, replace=False).astype(np.int32)
+    q = rng.choice([-2, -1, 1, 3], n).astype(np.int32)
+    tgt = rng.integers(0, sites, t).astype(np.int32)
+    with lgm.Coulomb(*dims, cutoff=cutoff, path=path) as ctx:
+        last = len(ctx.variants()) - 1
+        got = ctx.potentials(src, q, tgt)
+        assert ctx.last_launch()["variant"] == (32 if tile else last)
+        d = [torch.as_tensor(a).cuda() for a in (src, q, tgt)]
+        out = torch.zeros(t, dtype=torch.float64, device="cuda")
+        stream, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=stream):
+            ctx.potentials_async(d[0].data_ptr(), d[1].data_ptr(), n, d[2].data_ptr(), 5000,
+                                 out.data_ptr(), stream=stream.cuda_stream)
+        g.replay()
+        torch.cuda.synchronize()
+        few = out[:5000].cpu().numpy()
+        ctx.set_variant(last if tile else 32)
+        other = ctx.potentials(src, q, tgt)
+        norm = ctx.potentials(src, np.abs(q), tgt)
+    # FP64 sums of at most n terms or runs, rounded n times each
+    assert np.all(np.abs(got - other) <= 2 * n * 2.0 ** -53 * norm)
+    assert np.all(np.abs(few - got[:5000]) <= 2 * n * 2.0 ** -53 * norm[:5000])
