@@ -248,9 +248,12 @@ lgm_status lgm_set_counting(lgm_ctx* ctx, int32_t enable);
  * pairs per thread, FP32 run length).  lgm_autotune times each on synthetic
  * charges of the given size (n sources, t targets, `terms`) with CUDA events,
  * remembers the fastest for that size bucket (half-octaves of targets and
- * source chunks) on this context, and reports it; calls in an untuned bucket
- * use the last variant, or one kernel when they have few sources (up to 512, or
- * 1024 and 2^25 pairs, or 2048 and 2^22 pairs).  It allocates, so call it before any stream capture. */
+ * source chunks) on this context, and reports it.  Calls in an untuned bucket
+ * use the last variant (with tables and many targets variant 32), or one kernel
+ * when they have few sources: up to 512, or 1024 and 2^25 pairs, or 2048 and 2^22
+ * pairs.  Where one kernel would serve the call it is timed too; if it wins,
+ * nothing is remembered and the last variant is reported.  Allocates: call it
+ * before any stream capture. */
 lgm_status lgm_autotune(lgm_ctx* ctx, lgm_kind kind, uint32_t terms, int32_t n, int32_t t,
                         int32_t* chosen);
 /* Force a variant (0 .. lgm_variant_count()-1) for every call, -1 = automatic. */

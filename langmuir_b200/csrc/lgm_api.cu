@@ -976,17 +976,24 @@ SmallFn small_fn(int kind, int path) {
 
 // A call of few sources takes the one-kernel form (lgm_small.cuh): up to
 // kSmallSources of them and small_pairs unculled pairs, where the chain's
-// launches cost more than the pairs it culls, with no variant forced or tuned
-// for the size (the FP64 precision has none), no pair counting, and a table
-// that leaves two CTAs their shared memory.
+// launches cost more than the pairs it culls, and a table that leaves two CTAs
+// their shared memory.
+bool small_fits(const lgm_ctx* c, int kind, const Shape& sh, int n, int t, bool all_sites) {
+    const bool fp64_terms = sum_path(c) == LGM_PATH_TABLE64;
+    return n >= 1 && n <= kSmallSources &&
+           (long long)n * t * sh.nterms <= small_pairs(n, fp64_terms, all_sites) &&
+           small_smem(n, small_table(c, kind), fp64_terms ? 8 : 4) <= kSmallSmem;
+}
+
+// It does so with no variant forced, no pair counting, and none tuned for the size
+// (the FP64 precision has none).  The tuner tries the form where it would serve a
+// call with given targets: there its choice stands.
 bool small_call(const lgm_ctx* c, int kind, const Shape& sh, int n, int t, bool all_sites) {
-    const bool f64 = c->cfg.precision == LGM_PREC_FP64, fp64_terms = sum_path(c) == LGM_PATH_TABLE64;
+    const bool f64 = c->cfg.precision == LGM_PREC_FP64;
     if (f64 ? !f64_table(c) : c->forced_variant >= 0 || c->counting) return false;
-    if (n < 1 || n > kSmallSources ||
-        (long long)n * t * sh.nterms > small_pairs(n, fp64_terms, all_sites))
-        return false;
-    if (!f64 && c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks))) return false;
-    return small_smem(n, small_table(c, kind), fp64_terms ? 8 : 4) <= kSmallSmem;
+    if (!small_fits(c, kind, sh, n, t, all_sites)) return false;
+    return f64 || !c->tune_cache.count(tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks)) ||
+           !small_fits(c, kind, sh, n, t, false);
 }
 
 // flag: null, or the host-visible word the last CTA writes {call, error} to.
@@ -1070,14 +1077,17 @@ lgm_status launch_potentials(lgm_ctx* c, int kind, unsigned terms, const int32_t
     const int v = f64 ? kDefaultVariant : choose_variant(c, kind, sh, n);
     const int fmt = direct || !kVariants[v].tc ? kFmtFloat : kFmtHalf;
     lgm_status s;
-    // an untuned call with tables makes room for both default variants: a smaller
-    // one may take the other
-    const bool both = !f64 && cf.path != LGM_PATH_RSQRT && c->forced_variant < 0;
+    // room for every variant that a smaller call may take: with tables both
+    // defaults, and those that were tuned
     std::vector<int> vs = {direct ? kDirect : v};
-    if (both) vs = {v, kDefaultVariant, kTileVariant};
-    if ((s = lay_out(c, sh, n, t, both ? kFmtFloat | kFmtHalf : fmt, fn_index(kind, sum_path(c)), vs)) !=
-        LGM_OK)
-        return s;
+    int room = fmt;
+    if (!f64 && c->forced_variant < 0 && (cf.path != LGM_PATH_RSQRT || !c->tune_cache.empty())) {
+        room = kFmtFloat | kFmtHalf;
+        vs.push_back(kDefaultVariant);
+        if (cf.path != LGM_PATH_RSQRT) vs.push_back(kTileVariant);
+        for (const auto& tuned : c->tune_cache) vs.push_back(tuned.second);
+    }
+    if ((s = lay_out(c, sh, n, t, room, fn_index(kind, sum_path(c)), vs)) != LGM_OK) return s;
     if ((s = prep(c, terms, d_src, d_q, n, d_tgt_site, t, all_sites, sh, fmt, st)) != LGM_OK)
         return s;
     int splits = 1;
@@ -1583,11 +1593,42 @@ lgm_status lgm_autotune(lgm_ctx* c, lgm_kind kind, uint32_t terms, int32_t n, in
         std::sort(ms, ms + 3);
         if (ms[1] < best_ms) { best_ms = ms[1]; best = v; }
     }
+    // Where the one-kernel form would serve the call, it is timed against the whole
+    // chain of the fastest variant; if it wins, no variant is remembered.
+    bool one_kernel = false;
+    const uint64_t key = tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks);
+    if (s == LGM_OK && c->cfg.precision != LGM_PREC_FP64 && small_fits(c, kind, sh, n, t, false) &&
+        (s = grow_device(c, &c->d_o, &c->o_cap, (size_t)t)) == LGM_OK) {
+        const int forced = c->forced_variant;
+        const bool counting = c->counting, timing = c->timing;
+        c->counting = c->timing = false;
+        c->tune_cache.erase(key);
+        float form_ms[2] = {0.f, 0.f};
+        for (int form = 0; form < 2 && s == LGM_OK; ++form) {
+            c->forced_variant = form == 0 ? best : -1;
+            float ms[3];
+            for (int r = -1; r < 3 && s == LGM_OK; ++r) {  // the first to warm up
+                cudaEventRecord(e0, st);
+                s = launch_potentials(c, kind, terms, c->d_s, c->d_q, n, c->d_t, t, 0, c->d_o, st);
+                cudaEventRecord(e1, st);
+                cudaEventSynchronize(e1);
+                if (r >= 0) cudaEventElapsedTime(&ms[r], e0, e1);
+            }
+            if (s != LGM_OK) break;
+            std::sort(ms, ms + 3);
+            form_ms[form] = ms[1];
+        }
+        c->forced_variant = forced;
+        c->counting = counting;
+        c->timing = timing;
+        one_kernel = form_ms[1] <= form_ms[0];
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (s != LGM_OK) return s;
     if ((s = check_device_error(c, st)) != LGM_OK) return s;
-    c->tune_cache[tune_key(kind, c->cfg.path, sh.t_phys, sh.n_chunks)] = best;
+    if (one_kernel) best = kDefaultVariant;
+    else c->tune_cache[key] = best;
     if (chosen) *chosen = best;
     return LGM_OK;
 }

@@ -48,3 +48,31 @@ def test_every_site(lgm, n, path, one):
         chain = ctx.kernel1(src, q)
         norm = ctx.kernel1(src, np.abs(q))
     assert np.all(np.abs(got - chain) <= 1e-13 * norm)
+
+
+def test_tuning_knows_the_one_kernel_form(lgm):
+    """163 sources and targets: one kernel is far below half the chain's time, so tuning
+    the size must not move it to the chain; nor every-site calls, which tuning does not
+    time.  Larger sizes keep the variant found."""
+    dims = (64, 61, 30)
+    V = 64 * 61 * 30
+    rng = np.random.default_rng(2)
+    src = rng.choice(V, 3000, replace=False).astype(np.int32)
+    q = rng.choice([-1, 1], 3000).astype(np.int32)
+    with lgm.Coulomb(*dims, cutoff=15) as ctx:
+        last = len(ctx.variants()) - 1
+        before = ctx.potentials(src[:163], q[:163], src[:163])
+        assert ctx.autotune(163, 163) == last
+        np.testing.assert_array_equal(ctx.potentials(src[:163], q[:163], src[:163]), before)
+        assert ctx.last_launch()["kernel_launches"] == 1
+        ctx.autotune(1000, V)
+        ctx.kernel1(src[:1000], q[:1000])
+        assert ctx.last_launch()["kernel_launches"] == 1
+        best = ctx.autotune(3000, 3000)
+        ctx.potentials(src, q, src)
+        assert ctx.last_launch()["variant"] == best
+        # a tuned context keeps the settings it had
+        ctx.set_variant(0)
+        ctx.autotune(163, 163)
+        ctx.potentials(src[:163], q[:163], src[:163])
+        assert ctx.last_launch()["variant"] == 0
