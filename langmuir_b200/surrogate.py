@@ -195,8 +195,18 @@ def _aligned(t, nbytes):
 
 def _masters(params):
     """The twelve FP32 masters as contiguous, 16-byte aligned tensors and a C array of their
-    pointers."""
-    ps = [_aligned(p.float(), 16) for p in params]
+    pointers.  The kernels read every entry, so a tensor short of entries is refused; the first
+    layer's may be broadcast to its shape, as in conv_weights_bf16, and no other shape."""
+    ps = []
+    for p, (name, shape) in zip(params, PARAM_SHAPES, strict=True):
+        if p.shape != shape:
+            if name == "c1w":
+                full = torch.empty(shape, device=p.device)
+                full[:] = p
+                p = full
+            elif p.numel() < math.prod(shape):
+                raise ValueError(f"{name}: {tuple(p.shape)} holds less than {shape}")
+        ps.append(_aligned(p.float(), 16))
     return ps, (_vp * len(ps))(*[p.data_ptr() for p in ps])
 
 
