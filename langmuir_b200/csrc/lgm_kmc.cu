@@ -1383,8 +1383,16 @@ __device__ __forceinline__ void step_class_sum(const float4* src, int n, float q
     }
 }
 
-// The block advances replica G by `steps` steps.
-template <int NT>
+// Carriers of a species up to which contested sites and a site's hole are looked
+// up in the list itself.  That is quadratic: past it they are claimed and mapped
+// in the replica's global arrays, as the separate kernels do.  (us a step, 64
+// replicas without Coulomb sums, list and arrays: 1966 holes 85 and 32, 490 11 and
+// 8; with sums, 490 carriers of both kinds 42.3 and 40.6.)
+constexpr int kListMost = 128;
+
+// The block advances replica G by `steps` steps.  COUL: with Coulomb sums, where
+// the replica has them.
+template <int NT, bool COUL>
 __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb, int win) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ double2 red[32];
@@ -1421,6 +1429,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
     }
     __syncthreads();
     const Dev& D = sD;
+    const bool coulomb = COUL && D.coulomb;
     const int nd = D.dq != 0 ? D.nd : 0;
     if (local) {
         for (int i = tid; i < s_cnt[I_NE]; i += NT) sA.es[i] = G.e_site[i];
@@ -1429,7 +1438,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
     }
     // charged defects stay where they are: their records once, behind the carriers'
     float4* sd = G.geo + G.cap_e + G.cap_h;
-    if (D.coulomb)
+    if (coulomb)
         for (int i = tid; i < nd; i += NT) sd[i] = step_record(D, D.defects[i]);
     __syncthreads();
 
@@ -1468,7 +1477,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                 f = nb[uint_below(r.w[0], (uint32_t)m)];
             }
             (e ? A.ef : A.hf)[k] = f;
-            if (D.coulomb)
+            if (coulomb)
                 (e ? A.se : A.sh)[k] =
                     make_float4(-2.f * x, -2.f * y, -2.f * z, (float)(x * x + y * y + z * z) - 0.5f);
         }
@@ -1484,7 +1493,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
         __syncthreads();
         // ---- potentials and decisions (decide_body): `split` threads per carrier
         int split = 1;
-        while (D.coulomb && split < 8 && 2 * split * n <= NT) split *= 2;
+        while (coulomb && split < 8 && 2 * split * n <= NT) split *= 2;
         const int part = tid & (split - 1);
         for (int c0 = 0; c0 < n; c0 += NT / split) {
             const int i = c0 + tid / split;
@@ -1502,13 +1511,13 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
             double dpot = 0.0, b1 = 0.0, b2 = 0.0;
             if (on && type == T_EMPTY && part == 0) {
                 dpot = D.pot[f] - D.pot[site];
-                if (D.coulomb) {
+                if (coulomb) {
                     b1 = binding(D, e, site);
                     b2 = binding(D, e, f);
                 }
             }
             double V[2] = {0.0, 0.0}, M[2] = {0.0, 0.0};
-            if (D.coulomb) {  // (a target that is not empty needs no potential)
+            if (coulomb) {  // (a target that is not empty needs no potential)
                 if (on && type == T_EMPTY) {
                     const unsigned ulim = __float_as_uint((float)D.cutoff2 - 0.5f);
                     int xa, ya, za, xb, yb, zb;
@@ -1554,7 +1563,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                 const Philox4 r = draw(D, step, (uint32_t)k, e ? RNG_DECIDE_E : RNG_DECIDE_H);
                 const double u = unit_double(r.w[0], r.w[1]);
                 double pd = dpot * q;
-                if (D.coulomb) {
+                if (coulomb) {
                     const double p1 = D.prefactor * V[0] + b1;
                     const double p2 = D.prefactor * V[1] - D.sI100 * q + b2;
                     de = q * (p2 - p1);
@@ -1614,6 +1623,11 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
         if (nflag > 0) __syncthreads();
         // ---- recombination (recomb_*_body); a hole's index by looking its site up
         if (recomb) {
+            const bool hole_map = nh > kListMost;
+            if (hole_map) {
+                for (int i = tid; i < nh; i += NT) D.h_at[A.hs[i]] = i;
+                __syncthreads();
+            }
             for (int i = tid; i < ne; i += NT) {
                 const int site = A.es[i];
                 int at = -1, cnt = 0;
@@ -1653,7 +1667,9 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                     if (cnt > 0) at = cand[uint_below(r.w[0], (uint32_t)cnt)];
                 }
                 int hk = -1;
-                if (at >= 0)
+                if (at >= 0 && hole_map)
+                    hk = D.h_at[at];
+                else if (at >= 0)
                     for (int j = 0; j < nh; ++j)
                         if (A.hs[j] == at) hk = j;
                 A.rch[i] = hk;
@@ -1674,9 +1690,23 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
             __syncthreads();
             for (int i = tid; i < ne; i += NT)
                 if (A.rch[i] >= 0) A.rcl[A.rch[i]] = INT_MAX;
+            if (hole_map) {
+                for (int i = tid; i < nh; i += NT) D.h_at[A.hs[i]] = -1;
+                __syncthreads();  // a hole's site is read before it leaves
+            }
         }
         // ---- completeTick in list order (claim_body, move_body): the lowest
         // index among a species' accepted moves to a site takes it
+        const bool claims = max(ne, nh) > kListMost;
+        if (claims) {
+            for (int i = tid; i < n; i += NT) {
+                const bool e = i < ne;
+                const int k = e ? i : i - ne, f = (e ? A.ef : A.hf)[k];
+                if (f >= 0 && f < D.V) atomicMin(&(e ? D.claim_e : D.claim_h)[f], k);
+            }
+            __syncthreads();
+        }
+        int moved = 0;
         for (int i = tid; i < n; i += NT) {
             const bool e = i < ne;
             const int k = e ? i : i - ne;
@@ -1691,20 +1721,32 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                 sites[k] = -1;
                 s_cnt[I_REMOVED] = 1;
                 atomicMin(&s_cnt[e ? I_FIRST_E : I_FIRST_H], k);
-                if (f >= 0) atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
+                moved += f >= 0;
                 continue;
             }
             bool mine = true;
+            if (claims) {
+                mine = (e ? D.claim_e : D.claim_h)[f] == k;
+            } else {
 #pragma unroll 8
-            for (int j = 0; j < k; ++j) mine &= to[j] != f;
+                for (int j = 0; j < k; ++j) mine &= to[j] != f;
+            }
             if (mine) {
                 own[site] = T_EMPTY;
                 own[f] = e ? T_ELECTRON : T_HOLE;
                 sites[k] = f;
-                atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
+                ++moved;
             }
         }
+        moved = __reduce_add_sync(0xffffffffu, moved);
+        if ((tid & 31) == 0 && moved) atomicAdd(&s_ctr[C_ACCEPTED], (unsigned long long)moved);
         __syncthreads();
+        if (claims)  // (the proposals of the next step are a barrier away)
+            for (int i = tid; i < n; i += NT) {
+                const bool e = i < ne;
+                const int f = e ? A.ef[i] : A.hf[i - ne];
+                if (f >= 0 && f < D.V) (e ? D.claim_e : D.claim_h)[f] = INT_MAX;
+            }
         compact_inject_body(D, warp_sums, reinterpret_cast<double*>(red));
         __syncthreads();
     }
@@ -1718,16 +1760,17 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
 }
 
 // Block b advances replica list[b].  recomb: the batch's flag.
-template <int NT>
-__global__ void __launch_bounds__(NT, NT == 128 ? 4 : 2)
+// Without Coulomb sums a step is all latency, and twice the blocks fit an SM.
+template <int NT, bool COUL>
+__global__ void __launch_bounds__(NT, (COUL ? 512 : 1024) / NT)
 kb_fused(const Dev* R, const int* list, int steps, int recomb, int win) {
-    fused_steps<NT>(R[list[blockIdx.x]], steps, recomb, win);
+    fused_steps<NT, COUL>(R[list[blockIdx.x]], steps, recomb, win);
 }
 // A small standalone replica, one block.
 constexpr int kFusedAloneThreads = 512;
 __global__ void __launch_bounds__(kFusedAloneThreads)
 k_fused(const __grid_constant__ Dev D, int steps, int recomb, int win) {
-    fused_steps<kFusedAloneThreads>(D, steps, recomb, win);
+    fused_steps<kFusedAloneThreads, true>(D, steps, recomb, win);
 }
 
 // ---- host side -------------------------------------------------------------------
@@ -2699,6 +2742,8 @@ const int kChunksPerItem[] = {16, 48};
 // A batch whose replicas all have room for at most this many charges takes
 // the fused step by default (one block per replica).
 constexpr int kFusedMaxCharges = 2048;
+// Replicas without Coulomb sums: room for more charges takes blocks of 256 threads.
+constexpr int kFusedSmallCharges = 512;
 // The fused step's window, and the shared memory of an SM that its blocks share.
 constexpr int kStepWindow = 1024;
 constexpr int kStepSmem = 200 * 1024;
@@ -2846,13 +2891,14 @@ lgm_status enqueue_batch_pair(lgm_kmc_batch* b, cudaStream_t st) {
 }
 
 using FusedFn = void (*)(const Dev*, const int*, int, int, int);
-FusedFn fused_fn(int threads) {
-    return threads <= 128 ? kb_fused<128> : kb_fused<256>;
+FusedFn fused_fn(int threads, bool coulomb) {
+    if (coulomb) return threads <= 128 ? kb_fused<128, true> : kb_fused<256, true>;
+    return threads <= 128 ? kb_fused<128, false> : kb_fused<256, false>;
 }
 
 void launch_fused(const lgm_kmc_batch* b, cudaStream_t st, int steps) {
     const int n = (int)b->fused.size();
-    fused_fn(b->fused_threads)<<<n, b->fused_threads, (size_t)b->fused_win * kStepBytes, st>>>(
+    fused_fn(b->fused_threads, b->coulomb)<<<n, b->fused_threads, (size_t)b->fused_win * kStepBytes, st>>>(
         b->d_reps, b->d_fused, steps, b->recomb, b->fused_win);
 }
 
@@ -2984,13 +3030,26 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
         const int per_sm = ((int)b->fused.size() + b->reps[0]->sm_count - 1) / b->reps[0]->sm_count;
         int cap = 1;
         for (int r : b->fused) cap = std::max({cap, b->hD[r].cap_e, b->hD[r].cap_h});
-        b->fused_win = std::max(128, std::min({cap + 2, kStepWindow,
-                                               kStepSmem / per_sm / kStepBytes}));
         // Up to two blocks an SM 256 threads are the faster ones (200 replicas of
         // 128x128: 18 us a step against 22), beyond that 128 (1024: 62 against 72).
         b->fused_threads = per_sm <= 2 ? 256 : 128;
+        // Without Coulomb sums (1024 threads an SM) the size decides: 600 replicas of 60
+        // holes 4.7 us a step at 128 threads and 7.9 at 256, 900 of 490 carriers of each
+        // kind 91 and 41.
+        int resident = per_sm;
+        if (!b->coulomb) {
+            int room = 0;
+            for (int r : b->fused) room = std::max(room, b->hD[r].cap_e + b->hD[r].cap_h);
+            b->fused_threads = room > kFusedSmallCharges ? 256 : 128;
+            resident = std::min(per_sm, 1024 / b->fused_threads);
+        }
+        b->fused_win = std::max(128, std::min({cap + 2, kStepWindow,
+                                               kStepSmem / resident / kStepBytes}));
+        // ... and a window that cannot hold every replica leaves its memory to L1, for
+        // the global arrays (600 replicas of 1966 holes 107 us a step and 72).
+        if (!b->coulomb && b->fused_win < cap + 2) b->fused_win = 128;
         // the limit is the function's, not the batch's: always the largest window
-        const cudaError_t e = cudaFuncSetAttribute(fused_fn(b->fused_threads),
+        const cudaError_t e = cudaFuncSetAttribute(fused_fn(b->fused_threads, b->coulomb),
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    kStepWindow * kStepBytes);
         if (e != cudaSuccess) return bfail(b, LGM_ERR_CUDA, "shared memory of the fused step");
