@@ -980,8 +980,9 @@ SmallFn small_fn(int kind, int path) {
 // their shared memory.
 bool small_fits(const lgm_ctx* c, int kind, const Shape& sh, int n, int t, bool all_sites) {
     const bool fp64_terms = sum_path(c) == LGM_PATH_TABLE64;
+    const bool mufu = kind == LGM_POINT && sum_path(c) == LGM_PATH_RSQRT;
     return n >= 1 && n <= kSmallSources &&
-           (long long)n * t * sh.nterms <= small_pairs(n, fp64_terms, all_sites) &&
+           small_size(n, t, sh.nterms, fp64_terms, mufu, all_sites) &&
            small_smem(n, small_table(c, kind), fp64_terms ? 8 : 4) <= kSmallSmem;
 }
 

@@ -21,10 +21,12 @@ namespace lgm {
 
 constexpr int kSmallThreads = 256, kSmallWarps = kSmallThreads / 32;
 constexpr size_t kSmallSmem = 96 * 1024;  // dynamic shared memory, at most
-// Sources and unculled pairs of a call in this form, at most (small_pairs); its sort's
-// places in s_list and the index in its keys hold 2048.
+// Sources of a call in this form, at most: its sort's places in s_list and the index
+// in its keys hold 2048.
 constexpr int kSmallSources = 2048;
-inline long long small_pairs(int n, bool fp64, bool all_sites) {
+// The calls this form is the faster one for.  fp64: terms from FP64 tables; mufu: point
+// charges' from the MUFU.
+inline bool small_size(int n, long long t, int nterms, bool fp64, bool mufu, bool all_sites) {
     // The chain sorts the targets too, and culls; this form sorts the sources again in
     // every CTA, by counting up to 512 of them, in some microseconds more beyond that.
     // us a device call, this form and the chain, 256x256x16, cutoff 50:
@@ -32,10 +34,17 @@ inline long long small_pairs(int n, bool fp64, bool all_sites) {
     //   1024 sources, 2^24 pairs 28 and 31, 2^25 33 and 34, 2^27 77 and 61
     //   1500 sources, 2^22 pairs 31 and 30, 2^23 43 and 30; 2048, 2^22 34 and 30 (host
     //   call 55 and 54), 2^25 52 and 33
-    // Every site: a segment is a run along x and culls well; 1000 sources on 2^20 sites
-    // 139 and 204.  Terms from FP64 tables: 400 sources, 2^25 pairs 57 and 55.
-    if (!fp64 && n <= (all_sites ? 1024 : 512)) return 1ll << 62;
-    return n <= 1024 ? 1ll << 25 : 1ll << 22;
+    // FP64 terms: 512 sources, 2^25 pairs 46 and 46; 800, 2^23 36 and 33, 2^24 44 and 34;
+    //   1024, 2^22 25 and 32, 2^24 47 and 35.
+    // Every site: a segment is a run along x and culls well.  MUFU: 1024 sources on 2^20
+    //   sites 137 and 245, 2048 230 and 285 (cutoff 10 141 and 169), on 2^18 199 and 219
+    //   (108 and 100), on 2^14 51 and 36.  FP64 terms, 2^20 sites: 100 sources 110 and
+    //   197, 400 184 and 235 (the tile 187), 700 247 and 274 (the tile 229).
+    const long long pairs = n * t * nterms;
+    if (all_sites ? n <= (fp64 ? 400 : 1024) : n <= 512 && !fp64) return true;
+    if (all_sites && mufu && t >= 1ll << 19) return true;
+    if (n <= 512 || (n <= 1024 && !(fp64 && !all_sites))) return pairs <= 1ll << 25;
+    return pairs <= (n <= 1024 ? 1ll << 23 : 1ll << 22);
 }
 
 struct SmallArgs {
