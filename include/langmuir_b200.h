@@ -286,7 +286,10 @@ lgm_status lgm_variant_flags(int32_t variant, int32_t* flags);
  * warp on items of its own 32 targets; its `target_pairs` reads 1. */
 /* Culled variants: source chunks per work item (at least; more when a
  * tile's live chunks exceed 32 items) and, warp-specialised, the stages of
- * the copy ring (0 otherwise); both 0 for the other variants. */
+ * the copy ring (0 otherwise); both 0 for the other variants and for the
+ * default, whose items hold 8 to 72 groups of 16 sources as the call's size
+ * asks (more when the 32 targets' live groups exceed 16 items, 8 in calls of
+ * more than 262,144 targets x terms). */
 lgm_status lgm_variant_items(int32_t variant, int32_t* chunks_per_item, int32_t* stages);
 
 #ifdef __cplusplus

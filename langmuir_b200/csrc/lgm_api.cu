@@ -527,10 +527,10 @@ struct Variant {
              &pair_kernel_culled_ws<0, 2, NW, RP, SUB, S, MINB>},                             \
             S                                                                                 \
     }
-// r^2 on the tensor cores: warps of 32 targets, items of about three chunks
+// r^2 on the tensor cores: warps of 32 targets, items by the call's size (mma_items)
 #define LGM_VARIANT_MMA                                                                      \
     Variant {                                                                                 \
-        kMmaThreads, 1, kGroup, 1, 1, kItemGroups / kGroupsPerChunk,                          \
+        kMmaThreads, 1, kGroup, 1, 1, 0,                                                      \
             {nullptr, nullptr, nullptr, nullptr},                                             \
             {&pair_kernel_mma<0, 0, kMmaTabPoint>, &pair_kernel_mma<1, 0, kMmaTabGauss>,      \
              &pair_kernel_mma<0, 1, 8>, &pair_kernel_mma<0, 2, 8>},                           \
