@@ -1,6 +1,6 @@
 // lgm_cnn_tc.cu -- the surrogate's 32 -> 32 channel 3x3 convolution on the
 // 5th-generation tensor cores: TMA tensor loads, tcgen05.mma with accumulators
-// in tensor memory, a two-stage pipeline.
+// in tensor memory, a three-stage pipeline.
 //
 // Implicit GEMM per 8x16 output tile: M = 128 pixels, N = 32 output channels,
 // K = 9 taps x 32 input channels, issued as 18 UMMA instructions of
@@ -40,13 +40,12 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <cuda.h>
 #include <cudaTypedefs.h>
 
 #include <algorithm>
 
 #include "langmuir_b200_cnn.h"
-#include "lgm_device.cuh"
+#include "lgm_tcgen05.cuh"
 
 namespace {
 
@@ -70,74 +69,8 @@ constexpr uint32_t WS_BYTES = 9u * C8 * COUT * 16u;        // 18432
 constexpr uint32_t SMEM_BYTES = XS_BYTES + WS_BYTES + 128; // + mbarriers and TMEM slot
 constexpr uint32_t TMEM_COLS = 128;                        // NST stages of 32 columns (power of 2)
 
-// Instruction descriptor of tcgen05.mma kind::f16: D FP32 (bits 4-5 = 1),
-// A and B BF16 (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bit 17,
-// M >> 4 at bit 24.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COUT >> 3) << 17) |
-                            ((uint32_t)(128 >> 4) << 24);
-
-// Shared-memory matrix descriptor, no swizzle: start address, leading
-// (K-direction) and stride (M/N-direction) byte offsets in 16-byte units,
-// descriptor version 1 at bit 46.
-// layout: 0 no swizzle, 4 the 64-byte swizzle (bits 61-63).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo,
-                                              uint32_t layout = 0) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46) |
-           ((uint64_t)(layout & 7u) << 61);
-}
-
-// One TMA box of the 4-D NHWC tensor map into shared memory, completion
-// counted on `bar` (no multicast).
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1,
-                                            int c2, int c3, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-        "r"(smem_addr(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(da), "l"(db), "r"(kIdesc), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_addr(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void fence_before_sync() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void fence_after_sync() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-          "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-          "=r"(r[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
+constexpr uint32_t kIdesc = lgm::umma_idesc_bf16(128, COUT);
+constexpr uint64_t kSwizzle64 = 4ull << 61;  // the 64-byte layout in a matrix descriptor
 
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
@@ -145,10 +78,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 
 __device__ unsigned g_tc_error = 0;  // DEVERR_* bits of the tensor-core conv
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
 
 // Bounded wait that returns false after a timeout (and records it).
 __device__ __forceinline__ bool wait(uint64_t* bar, int use) {
@@ -175,13 +104,7 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
     const int ntiles = B * tiles_x * tiles_y;
     const int n = ((int)blockIdx.x < ntiles) ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         smem_addr(tslot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
+    if (warp == 0) lgm::tmem_alloc(tslot, TMEM_COLS);
     if (tid == 0) {
         for (int i = 0; i < 2 * NST; ++i) lgm::mbar_init(&full[i], 1);       // full, done
         for (int i = 2 * NST; i < 3 * NST; ++i) lgm::mbar_init(&full[i], 4);  // empty: a lane per
@@ -196,9 +119,9 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
             *reinterpret_cast<const uint4*>(w + (size_t)o * 9 * CIN + t * CIN + c8 * 8);
     }
     lgm::fence_proxy_async_smem();  // generic-proxy writes -> the tensor core's reads
-    fence_before_sync();
+    lgm::tc_fence_before();
     __syncthreads();
-    fence_after_sync();
+    lgm::tc_fence_after();
     const uint32_t tmem = *tslot;
     const uint32_t xs_a = smem_addr(smem), ws_a = smem_addr(ws);
 
@@ -222,8 +145,8 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
                 lgm::mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
 #pragma unroll 1
                 for (int kx = 0; kx < 3; ++kx)
-                    tma_load_4d(xs_a + st * STAGE_BYTES + kx * COPY_BYTES, &xmap, 0, x0 + kx - 1,
-                                y0 - 1, b, &full[st]);
+                    lgm::tma_box_4d(xs_a + st * STAGE_BYTES + kx * COPY_BYTES, &xmap, 0, x0 + kx - 1,
+                                    y0 - 1, b, &full[st]);
                 ++tma_issued;
             };
             for (int k = 0; k < NST && k < n; ++k) issue_tma(k);
@@ -232,7 +155,7 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
                 // the patch has landed; the epilogue has released the TMEM stage (tile k-NST)
                 ok = wait(&full[st], k / NST) && (k < NST || wait(&empty[st], (k - NST) / NST));
                 if (!ok) break;
-                fence_after_sync();
+                lgm::tc_fence_after();
                 const uint32_t xa = xs_a + st * STAGE_BYTES, d = tmem + (uint32_t)(st * 32);
 #pragma unroll 1
                 for (int t = 0; t < 9; ++t) {
@@ -241,14 +164,15 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
                     for (int j = 0; j < 2; ++j) {
                         // A: rows 16 ky .. 16 ky + 127 of copy kx, channels 16j .. 16j+15
                         const uint64_t da =
-                            smem_desc(xa + kx * COPY_BYTES + ky * TX * 64 + j * 32, 16, 512, 4);
+                            lgm::umma_desc(xa + kx * COPY_BYTES + ky * TX * 64 + j * 32, 16, 512) |
+                            kSwizzle64;
                         // B: 32 output channels of tap t, the same 16 channels
-                        const uint64_t db =
-                            smem_desc(ws_a + (uint32_t)(((t * C8 + 2 * j) * COUT) * 16), COUT * 16, 128);
-                        umma(d, da, db, (t | j) ? 1u : 0u);
+                        const uint64_t db = lgm::umma_desc(
+                            ws_a + (uint32_t)(((t * C8 + 2 * j) * COUT) * 16), COUT * 16, 128);
+                        lgm::umma_f16(d, da, db, kIdesc, (t | j) ? 1u : 0u);
                     }
                 }
-                umma_commit(&done[st]);
+                lgm::umma_commit_to(&done[st]);
                 ++mma_issued;
                 // tile k-1's MMAs finished -> its patch buffer takes tile k-1+NST
                 if (k >= 1 && k - 1 + NST < n) {
@@ -275,12 +199,12 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
         for (int k = g; k < n; k += 2) {
             const int st = k % NST;
             if (!wait(&done[st], k / NST)) break;
-            fence_after_sync();
+            lgm::tc_fence_after();
             float v[32];
-            tmem_ld32(tmem + (uint32_t)(st * 32) + ((uint32_t)(wq * 32) << 16), v);
-            fence_before_sync();
+            lgm::tmem_ld32x(tmem + (uint32_t)(st * 32) + ((uint32_t)(wq * 32) << 16), v);
+            lgm::tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[st]);  // this warp's TMEM lanes are read
+            if (lane == 0) lgm::mbar_arrive(&empty[st]);  // this warp's TMEM lanes are read
             int b, y0, x0;
             origin(k, b, y0, x0);
             // this thread's pixel: tile row 2*wq + lane/16, column lane%16
@@ -319,13 +243,10 @@ conv3x3_fwd_tc(const __grid_constant__ CUtensorMap xmap, const bf16* __restrict_
             }
         }
     }
-    fence_before_sync();
+    lgm::tc_fence_before();
     __syncthreads();
-    fence_after_sync();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                     "r"(TMEM_COLS)
-                     : "memory");
+    lgm::tc_fence_after();
+    if (warp == 0) lgm::tmem_free(tmem, TMEM_COLS);
 }
 
 }  // namespace
