@@ -84,15 +84,16 @@ lgm_status lgm_cnn_to_bf16(const float* in, void* out, int32_t n, const float* r
  * (FP32 masters in; the BF16 roundings of the layer-by-layer kernels).
  * params[12]: c1w [32][9], c1b, c2w [32][288], c2b, c3w, c3b, c4w, c4b,
  * f1w [64][32], f1b, f2w [2][64], f2b; c2w, c3w and c4w 16-byte aligned.
- * x: [B][H][W] BF16, 4-byte aligned, H % 16 == 0, W % 64 == 0; y: [B][2] FP32.  saved: device memory of lgm_cnn_net_bytes(B, H,
- * W, keep) bytes, 256-byte aligned; with keep != 0 it holds what the backward
- * call reads. */
+ * x: [B][H][W] BF16, 4-byte aligned, H % 16 == 0, W % 64 == 0; y: [B][2] FP32.
+ * saved: device memory of lgm_cnn_net_bytes(B, H, W, keep) bytes, 256-byte
+ * aligned; with keep != 0 it holds what the backward call reads. */
 size_t lgm_cnn_net_bytes(int32_t B, int32_t H, int32_t W, int32_t which);
 lgm_status lgm_cnn_net_forward(const void* x, const float* const* params, void* saved, float* y,
                                int32_t B, int32_t H, int32_t W, int32_t keep, void* stream);
 
 /* The gradients of the twelve parameters from dL/dy [B][2] (overwritten, each
- * 16-byte aligned), after a forward call with keep != 0 on the same x.  work: lgm_cnn_net_bytes(B, H, W, 2) bytes, 256-byte aligned. */
+ * 16-byte aligned), after a forward call with keep != 0 on the same x.  work:
+ * lgm_cnn_net_bytes(B, H, W, 2) bytes, 256-byte aligned. */
 lgm_status lgm_cnn_net_backward(const void* x, const void* saved, const float* dy, void* work,
                                 float* const* grads, int32_t B, int32_t H, int32_t W, void* stream);
 

@@ -94,8 +94,8 @@ __device__ __forceinline__ uint32_t half_mask(uint32_t m) { return (m & 0x10001u
 // (At 80 registers for three blocks it spilled and lost 2%; with 8 pixels in
 // flight instead of 16 half the gain was left.)
 // Bound: the ReLU/pool arithmetic, about 100 instructions per 1024 values (ALU
-// pipe half busy), then HBM (the pooled output of 1024 images, 41 us).  The
-// shared-memory tile of conv1_fwd took 242 us for 1024 images, the plain loop 120.
+// pipe 60% busy, issue slots 63%), then HBM (the pooled output of 1024 images, 41 us).
+// 1024 images: the shared-memory tile of conv1_fwd 234 us, the plain loop 120, now 106.
 constexpr int C1_WARPS = 8;
 constexpr int C1_CTAS = 2;  // an SM
 template <bool MASK>
@@ -350,8 +350,9 @@ __device__ __forceinline__ bool net_wait(uint64_t* bar, int use) {
 //              whose bit is set in bits [B][2H][2W] -> out planes [2H][2W]
 // w: FP32 masters [32][288], or with FLIP the same masters of the layer whose
 // input gradient this is (taps reversed, channels transposed).
-// Bound: the shared-memory reads of the A operand, 4 KB per multiplication (32
-// clocks where the tensor core takes 16), about 600 clocks a tile and SM.
+// Bound: the tensor core's reads of the A operand, 4 KB per multiplication of only 32
+// columns.  Layer 2, 1024 images: 121 us, 868 clocks a tile and SM, the tcgen05 pipe
+// busy in 89% of them (43 clocks a multiplication).
 template <int EP, bool FLIP>
 __global__ void __launch_bounds__(CONV_THREADS, 3)
 conv_planes(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ w,

@@ -1298,11 +1298,11 @@ __global__ void __launch_bounds__(kCompactThreads) kb_compact_inject(const Dev* 
 // goes on in its global arrays), a carrier's two potentials are summed and
 // decided by the same threads without a pass in between, and contested sites
 // are settled by comparing the accepted moves of the list instead of claiming
-// sites in memory.  1024 solar cells of 128x128 after 2000 steps of burn-in: 53 us
-// a step, with the phases as separate passes over global arrays 81.  At that load
-// the blocks issue 1.7 instructions a clock and an SM (MUFU 24%, FMA 21% busy):
-// carriers differ between replicas, and the SM with the most sets the time.
-// Holding 5-8 blocks an SM instead of 4 (fewer registers) changed nothing.
+// sites in memory.  1024 solar cells of 128x128, steps 2000 to 5000: 28 to
+// 34 us a step, with the phases as separate passes over global arrays 50 to 58.  At
+// that load the blocks issue 1.7 instructions a clock and an SM (MUFU 24%, FMA 21%
+// busy): carriers differ between replicas, and the SM with the most sets the time.
+// Holding 5-8 blocks an SM instead of 4 (fewer registers) gained nothing.
 //
 // It takes the separate kernels' decisions: the same draws, the same rules, FP32
 // runs of kSUB sources of one charge class in list order folded into FP64
@@ -2165,7 +2165,7 @@ constexpr int kFusedStepsPerLaunch = 1000;
 // time than the separate kernels' launches, some 40 us a step whatever the
 // size.  With 512 threads a step takes about 6 us and 0.12 us per 1000 carriers x
 // sources x terms (us a step, fused and separate: 20 holes 5.6 and 37, 163 holes
-// 10.7 and 38, 490 carriers 33 and 40; 326 with both images, 319k, 47 and 40);
+// 10.4 and 38, 490 carriers 33 and 40; 326 with both images, 319k, 47 and 40);
 // the Gaussian table makes a pair about 1.5 times as dear (458 carriers, 48 and
 // 46).  The room decides, not the carriers alive, so a replica keeps one form.
 // Culled replicas sum their sources in cell order and stay as they are.
@@ -3030,8 +3030,9 @@ lgm_status partition_batch(lgm_kmc_batch* b) {
         const int per_sm = ((int)b->fused.size() + b->reps[0]->sm_count - 1) / b->reps[0]->sm_count;
         int cap = 1;
         for (int r : b->fused) cap = std::max({cap, b->hD[r].cap_e, b->hD[r].cap_h});
-        // Up to two blocks an SM 256 threads are the faster ones (200 replicas of
-        // 128x128: 18 us a step against 22), beyond that 128 (1024: 62 against 72).
+        // Up to two blocks an SM 256 threads are the faster ones (296 solar cells of
+        // 128x128: 13.9 us a step against 18.8), beyond that 128 (400: 20.3 against
+        // 23.6, 1024: 30.7 against 42.2).
         b->fused_threads = per_sm <= 2 ? 256 : 128;
         // Without Coulomb sums (1024 threads an SM) the size decides: 600 replicas of 60
         // holes 4.7 us a step at 128 threads and 7.9 at 256, 900 of 490 carriers of each
