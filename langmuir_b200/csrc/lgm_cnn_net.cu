@@ -593,7 +593,7 @@ wgrad_planes(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
         const uint32_t s = smem_addr(smem) + st * WG_STAGE;
         lgm::mbar_arrive_expect_tx(&full[st], WG_STAGE);
         lgm::tma_box_4d(s, &xmap, (x0 - 1) * 8, y0 - 1, 0, b, &full[st]);
-        // rows past the image read zeros and add nothing
+        // rows past the image read zeros and are left out
         lgm::tma_box_4d(s + PATCH_B, &dmap, x0 * 8, y0, 0, b, &full[st]);
     };
     int copied = 0;
@@ -613,9 +613,14 @@ wgrad_planes(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ C
         ok = __all_sync(0xffffffffu, net_wait(&full[st], k / WG_ST));
         if (!ok) break;
         const uint32_t xs = smem_addr(smem) + st * WG_STAGE, ds = xs + PATCH_B;
+        const int tile = (int)blockIdx.x + k * (int)gridDim.x;
+        const int rows = H - tile / tiles_x % tiles_y * TY;  // of the image from the tile's first on
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int row = 4 * q + 2 * h;  // tile rows row, row + 1
+            const int row = 4 * q + 2 * h;  // tile rows row, row + 1 (H is even)
+            // Past the image dA is zero, but the row above is not: no gradient there
+            // does not stop an infinity.
+            if (row >= rows) continue;
             uint32_t a[2][4];
 #pragma unroll
             for (int i = 0; i < 2; ++i)  // a0, a1: planes 2i, 2i+1, pixels 0-7; a2, a3: 8-15
