@@ -2511,7 +2511,9 @@ static lgm_status kmc_create_impl(const lgm_params* pin, int32_t device, uint32_
     if ((st = upload_carriers(k, k->e0.data(), (int)k->e0.size(), k->h0.data(),
                               (int)k->h0.size())) != LGM_OK)
         return bail(st, k->err);
-    if (!pool && cudaDeviceSynchronize() != cudaSuccess) return bail(LGM_ERR_CUDA, "set-up");
+    // (the stream of the copies above, not the device: another thread may be capturing)
+    if (!pool && cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        return bail(LGM_ERR_CUDA, "set-up");
     k->wcfg = nullptr;  // the caller's arrays are not kept
     *out = k;
     return LGM_OK;
@@ -3179,7 +3181,8 @@ lgm_status lgm_kmc_batch_create(const lgm_params* params, int32_t count, int32_t
         if (s != LGM_OK) return bail(s, "replica " + std::to_string(i) + ": " + lgm_kmc_last_error(nullptr));
         b->reps.push_back(k);
     }
-    if (cudaDeviceSynchronize() != cudaSuccess) return bail(LGM_ERR_CUDA, "replica set-up");
+    if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        return bail(LGM_ERR_CUDA, "replica set-up");
     // one interaction kind and one cutoff-table layout per batch
     b->gauss = b->reps[0]->D.gauss;
     b->coulomb = b->reps[0]->D.coulomb;
