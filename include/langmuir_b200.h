@@ -251,8 +251,9 @@ lgm_status lgm_set_counting(lgm_ctx* ctx, int32_t enable);
  * source chunks) on this context, and reports it.  Calls in an untuned bucket
  * use the last variant (with tables and many targets variant 32), or one kernel
  * when they have few sources: up to 512, or 1024 and 2^25 pairs (FP64 terms 512
- * and 2^25, 1024 and 2^23), or 2048 and 2^22; on every site up to 1024 (FP64
- * terms 400), and 2048 point charges without tables on 2^19 sites or more.  Where one kernel would serve the call it is timed too; if it wins,
+ * and 2^25, 1024 and 2^23), or 2048 and 4736 targets; on every site up to 1024
+ * (FP64 terms 400), and 2048 point charges without tables on 2^19 sites or more.
+ * Where one kernel would serve the call it is timed too; if it wins,
  * nothing is remembered and the last variant is reported.  Allocates: call it
  * before any stream capture. */
 lgm_status lgm_autotune(lgm_ctx* ctx, lgm_kind kind, uint32_t terms, int32_t n, int32_t t,

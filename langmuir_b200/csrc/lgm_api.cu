@@ -918,8 +918,11 @@ lgm_status launch_pair(lgm_ctx* c, int kind, int path, int v, const Shape& sh, c
 //   table64, cutoff 100: 2000 and 4000 of 128x128x32 (2^22) 56 and 45; 2000 and
 //   16,000 (2^24) 70 and 76
 //   table, cutoff 150: 2000 and 4000 of 128x128x32 1.14 to 1.18 times faster by the
-//   latter; 2000 and 16,000 (2^24) 59 and 64; every site of 64x64x64, cutoff 50,
-//   2000 sources 323 and 335
+//   latter; 2000 and 16,000 (2^24) 59 and 64
+//   table, every site, 6000 sources: 64x64x64, cutoff 30 417 and 376, 50 743 and 769, 100
+//   840 and 990; 92x166x64, 30 747 and 600, 50 1407 and 1309, 70 2070 and 2056, 100 2659
+//   and 2888; 256x256x16, 70 938 and 916, 100 1452 and 1491: the cutoff against the
+//   lattice's mean side decides (a short one leaves few reads that only the vote skips)
 // With terms from the MUFU the tensor-core kernel is never more than 4% behind; but
 // its masks grow as targets x sources, twice as fast as the tile's lists, and are
 // left alone past 64 GB.
@@ -932,7 +935,8 @@ bool tile_faster(const lgm_ctx* c, const Shape& sh, int n) {
         inside *= std::min(1.0, 2.0 * cf.electrostatic_cutoff / side);
     if (cf.path == LGM_PATH_TABLE64)
         return sh.t_phys > 65536 || inside > (cf.electrostatic_cutoff > 60 ? 0x1p24 : 0x1p27);
-    return (cf.electrostatic_cutoff >= 40 && sh.t_phys > 200000) ||
+    const double side = std::cbrt((double)c->volume);
+    return (cf.electrostatic_cutoff >= 0.78 * side && sh.t_phys > 200000) ||
            (cf.electrostatic_cutoff > 110 && inside > 0x1p24);
 }
 

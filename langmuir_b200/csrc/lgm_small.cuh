@@ -32,8 +32,11 @@ inline bool small_size(int n, long long t, int nterms, bool fp64, bool mufu, boo
     // us a device call, this form and the chain, 256x256x16, cutoff 50:
     //   128 sources, 2^27 pairs 63 and 298; 512, 2^26 58 and 56, 2^27 72 and 85
     //   1024 sources, 2^24 pairs 28 and 31, 2^25 33 and 34, 2^27 77 and 61
-    //   1500 sources, 2^22 pairs 31 and 30, 2^23 43 and 30; 2048, 2^22 34 and 30 (host
-    //   call 55 and 54), 2^25 52 and 33
+    //   1500 sources, 2^23 pairs 43 and 30; 2048, 2^25 52 and 33
+    // Past 1024 sources the sort sets the time, and the line is one CTA an SM (148 segments
+    // of 32): 2000 sources, 4000 targets 32 and 30 (host call 59 and 60), 42 and 39 when
+    // each call is waited for, 18 and 19 a call with three streams at work (1260 sources,
+    // 2520 targets, three terms: 15 and 19), since one launch leaves room for the others'.
     // FP64 terms: 512 sources, 2^25 pairs 46 and 46; 800, 2^23 36 and 33, 2^24 44 and 34;
     //   1024, 2^22 25 and 32, 2^24 47 and 35.
     // Every site: a segment is a run along x and culls well.  MUFU: 1024 sources on 2^20
@@ -44,7 +47,7 @@ inline bool small_size(int n, long long t, int nterms, bool fp64, bool mufu, boo
     if (all_sites ? n <= (fp64 ? 400 : 1024) : n <= 512 && !fp64) return true;
     if (all_sites && mufu && t >= 1ll << 19) return true;
     if (n <= 512 || (n <= 1024 && !(fp64 && !all_sites))) return pairs <= 1ll << 25;
-    return pairs <= (n <= 1024 ? 1ll << 23 : 1ll << 22);
+    return n <= 1024 ? pairs <= 1ll << 23 : t <= 148 * kSeg;
 }
 
 struct SmallArgs {

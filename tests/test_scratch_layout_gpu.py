@@ -97,7 +97,8 @@ def test_smaller_calls_are_captured_after_a_larger_one(lgm, n, warm, sizes, prec
     ((64, 64, 32), 100, 2, 2100, 8100, True), ((64, 64, 32), 100, 1, 2100, 8100, False),
     ((64, 64, 32), 150, 1, 2100, 7900, False), ((64, 64, 32), 150, 1, 2100, 8100, True),
     ((64, 64, 32), 40, 1, 2100, 199900, False), ((64, 64, 32), 40, 1, 2100, 200100, True),
-    ((64, 64, 32), 39, 1, 2100, 200100, False), ((64, 64, 32), 150, 0, 2100, 250000, False)])
+    ((64, 64, 32), 39, 1, 2100, 200100, False), ((64, 64, 32), 150, 0, 2100, 250000, False),
+    ((100, 90, 64), 64, 1, 2100, 200100, False), ((100, 90, 64), 65, 1, 2100, 200100, True)])
 def test_which_kernel_sums_from_tables(lgm, dims, cutoff, path, n, t, tile):
     """Both sides of the lines between the two default kernels, which add the same FP32
     runs (or FP64 terms) in another order of FP64 sums; a smaller call on the same

@@ -16,7 +16,7 @@ def lgm():
 @pytest.mark.parametrize("n,t,path,one", [
     (512, 70000, 0, True), (513, 70000, 0, False), (513, 65000, 0, True), (512, 70000, 1, True),
     (512, 70000, 2, False), (512, 65536, 2, True), (1024, 32768, 0, True), (1024, 32769, 0, False),
-    (1025, 4093, 0, False), (1025, 4092, 0, True), (2048, 2048, 0, True), (2048, 2049, 0, False)])
+    (1025, 4737, 0, False), (1025, 4736, 0, True), (2048, 4736, 0, True), (2048, 4737, 0, False)])
 def test_both_sides_of_the_lines(lgm, n, t, path, one):
     dims = (40, 36, 9)
     V = 40 * 36 * 9
