@@ -1383,11 +1383,12 @@ __device__ __forceinline__ void step_class_sum(const float4* src, int n, float q
     }
 }
 
-// Carriers of a species up to which contested sites and a site's hole are looked
-// up in the list itself.  That is quadratic: past it they are claimed and mapped
-// in the replica's global arrays, as the separate kernels do.  (us a step, 64
-// replicas without Coulomb sums, list and arrays: 1966 holes 85 and 32, 490 11 and
-// 8; with sums, 490 carriers of both kinds 42.3 and 40.6.)
+// Without Coulomb sums: carriers of a species up to which contested sites and a
+// site's hole are looked up in the list itself.  That is quadratic: past it they are
+// claimed and mapped in the replica's global arrays, as the separate kernels do.  (us
+// a step, 64 replicas, list and arrays: 1966 holes 85 and 32, 490 11 and 8.)  With
+// sums, which are quadratic too, the list serves any length: 490 carriers of both
+// kinds 42 and 41, but 27 holes 5.13 a step alone and 5.28 in a kernel with both ways.
 constexpr int kListMost = 128;
 
 // The block advances replica G by `steps` steps.  COUL: with Coulomb sums, where
@@ -1623,7 +1624,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
         if (nflag > 0) __syncthreads();
         // ---- recombination (recomb_*_body); a hole's index by looking its site up
         if (recomb) {
-            const bool hole_map = nh > kListMost;
+            const bool hole_map = !COUL && nh > kListMost;
             if (hole_map) {
                 for (int i = tid; i < nh; i += NT) D.h_at[A.hs[i]] = i;
                 __syncthreads();
@@ -1697,7 +1698,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
         }
         // ---- completeTick in list order (claim_body, move_body): the lowest
         // index among a species' accepted moves to a site takes it
-        const bool claims = max(ne, nh) > kListMost;
+        const bool claims = !COUL && max(ne, nh) > kListMost;
         if (claims) {
             for (int i = tid; i < n; i += NT) {
                 const bool e = i < ne;
@@ -1721,6 +1722,7 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                 sites[k] = -1;
                 s_cnt[I_REMOVED] = 1;
                 atomicMin(&s_cnt[e ? I_FIRST_E : I_FIRST_H], k);
+                if (COUL && f >= 0) atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
                 moved += f >= 0;
                 continue;
             }
@@ -1735,11 +1737,14 @@ __device__ __forceinline__ void fused_steps(const Dev& G, int steps, int recomb,
                 own[site] = T_EMPTY;
                 own[f] = e ? T_ELECTRON : T_HOLE;
                 sites[k] = f;
+                if (COUL) atomicAdd(&s_ctr[C_ACCEPTED], 1ull);
                 ++moved;
             }
         }
-        moved = __reduce_add_sync(0xffffffffu, moved);
-        if ((tid & 31) == 0 && moved) atomicAdd(&s_ctr[C_ACCEPTED], (unsigned long long)moved);
+        if (!COUL) {
+            moved = __reduce_add_sync(0xffffffffu, moved);
+            if ((tid & 31) == 0 && moved) atomicAdd(&s_ctr[C_ACCEPTED], (unsigned long long)moved);
+        }
         __syncthreads();
         if (claims)  // (the proposals of the next step are a barrier away)
             for (int i = tid; i < n; i += NT) {
@@ -2165,7 +2170,7 @@ constexpr int kFusedStepsPerLaunch = 1000;
 // time than the separate kernels' launches, some 40 us a step whatever the
 // size.  With 512 threads a step takes about 6 us and 0.12 us per 1000 carriers x
 // sources x terms (us a step, fused and separate: 20 holes 5.6 and 37, 163 holes
-// 10.4 and 38, 490 carriers 33 and 40; 326 with both images, 319k, 47 and 40);
+// 10.7 and 38, 490 carriers 33 and 40; 326 with both images, 319k, 47 and 40);
 // the Gaussian table makes a pair about 1.5 times as dear (458 carriers, 48 and
 // 46).  The room decides, not the carriers alive, so a replica keeps one form.
 // Culled replicas sum their sources in cell order and stay as they are.
